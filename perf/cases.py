@@ -171,3 +171,75 @@ def tolerance(case):
     if kind == "sgd":
         return {"rel": 6e-3, "max": 2e-2}       # the same rounding of the weights; the momentum is float32
     return {"rel": 2e-2, "max": 0.2}            # chains of products rounded to bf16: 3e-3 to 1e-2
+
+
+# ---------------------------------------------------------------------------- the same in 64 bits
+
+def _swiglu_mlp(x, w_gu, w_down):
+    gate, up = (x @ w_gu.t()).chunk(2, -1)
+    return (torch.nn.functional.silu(gate) * up) @ w_down.t()
+
+
+def _stack(x, weights):
+    for w_gu, w_down in weights:
+        x = x + _swiglu_mlp(x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6), w_gu, w_down)
+    return x
+
+
+def _experts(x, logits, w_gu, w_down):
+    """Top-2 routing with the softmax of the two winners as gate weights; ``w_gu`` and ``w_down`` are per expert."""
+    top, idx = logits.topk(2, -1)
+    gates = top.softmax(-1)
+    out = torch.zeros_like(x)
+    for e in range(logits.shape[1]):
+        token, slot = (idx == e).nonzero(as_tuple=True)
+        if token.numel():
+            y = _swiglu_mlp(x[token], w_gu[e], w_down[e])
+            out = out.index_add(0, token, y * gates[token, slot].unsqueeze(1))
+    return out
+
+
+def exact(case, seed):
+    """What :func:`run` returns, by plain torch in float64 from the inputs that :func:`prepare` makes."""
+    if work(case)["flops"] > 1.5e14:  # too long on one GPU
+        return None
+    kind, s = case["kind"], prepare(case, seed)
+    if kind == "gemm":
+        a, b = s["a"].double(), s["b"].double()
+        out = (a.t() if case["a_mn"] else a) @ (b if case["b_mn"] else b.t())
+        return out if s["out"] is None else out + s["out"].double()
+    if kind == "sgd":
+        w, h = s["w"].double(), s["hyper"]
+        step = s["g"].double() + h["weight_decay"] * w
+        if s["m"] is None:
+            return {"w": w - h["lr"] * step, "m": None}
+        m = h["momentum"] * s["m"].double() + step
+        return {"w": w - h["lr"] * m, "m": m}
+    model, x = s["model"], s["x"].double()
+    lr = model.cfg.lr
+    if kind in ("mlp_step", "mlp_forward"):
+        weights = [[l.w_gu.double(), l.w_down.double()] for l in model.layers]
+        del s, model
+        if kind == "mlp_forward":
+            return _stack(x, weights)
+        flat = [w.requires_grad_() for pair in weights for w in pair]
+        out = _stack(x, weights)
+        loss = out.pow(2).mean()
+        grads = torch.autograd.grad(loss, flat)
+        with torch.no_grad():
+            new = [w.detach() - lr * g for w, g in zip(flat, grads)]
+        pairs = lambda v: [list(v[i:i + 2]) for i in range(0, len(v), 2)]  # noqa: E731
+        return {"loss": loss.detach().view(1), "weights": pairs(new), "grads": pairs(grads)}
+    experts, hidden = case["experts"], case["hidden"]
+    logits = s["logits"].double()
+    w_gu, w_down = model.w_gu.double(), model.w_down.double()
+    del s, model
+    per = lambda w_gu, w_down: (w_gu.view(experts, -1, hidden), w_down.view(experts, hidden, -1))  # noqa: E731
+    if kind == "moe_forward":
+        return _experts(x, logits, *per(w_gu, w_down))
+    wanted = [t.requires_grad_() for t in (x, logits, w_gu, w_down)]
+    out = _experts(x, logits, *per(w_gu, w_down))
+    loss = out.pow(2).mean()
+    dx, dlogits, g_gu, g_down = torch.autograd.grad(loss, wanted)
+    return {"loss": loss.detach().view(1), "out": out.detach(), "dx": dx, "dlogits": dlogits,
+            "weights": [w_gu.detach() - lr * g_gu, w_down.detach() - lr * g_down], "grads": [g_gu, g_down]}
