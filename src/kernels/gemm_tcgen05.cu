@@ -75,6 +75,9 @@ constexpr int PUSH_STAGING_BYTES = 8 * PUSH_WARP_BYTES;  // up to eight epilogue
 // in the wide variant (eight epilogue warps), four per warp otherwise.
 constexpr int OUT_STAGING_BYTES = 16 * 2048;
 
+constexpr int BAR_BYTES = 256;
+constexpr int MAX_ROW_TILES = 704;  // entries of the row-tile list: what shared memory leaves beside the ring
+
 template <int EPI>
 constexpr int staging_for() {
     return (EPI == EPI_PUSH || EPI == EPI_STORE_ROWS) ? PUSH_STAGING_BYTES : OUT_STAGING_BYTES;
@@ -85,8 +88,8 @@ constexpr int stages_for() {
 }
 template <int MODE, int EPI>
 constexpr int smem_for() {
-    return stages_for<MODE, EPI>() * Cfg<MODE>::STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/ +
-           staging_for<EPI>();
+    return stages_for<MODE, EPI>() * Cfg<MODE>::STAGE_BYTES + 1024 /*align slack*/ + BAR_BYTES +
+           2 * MAX_ROW_TILES + staging_for<EPI>();
 }
 
 struct KParams {
@@ -124,12 +127,22 @@ struct Tile {
     int b_row;     // K-major B: first row; MN-major B: added to the k coordinate
     int k0;        // first k
     int k_blocks;  // 64-wide k steps; 0 = write zeros
+    int rows;      // rows of the tile that exist (and, in a grouped problem, belong to its group)
     long d_row0;   // first output row
     bool skip;     // nothing to do (padding block of a grouped problem)
 };
 
+// Row blocks of a grouped problem on a tile of more than 128 rows: consecutive 128-row blocks of
+// one group are put together, up to a full tile; padding blocks are left out.  One entry per tile
+// row: first block | (blocks - 1) << 14.
+struct RowTiles {
+    const uint16_t* list;  // null = tile rows are TILE_M rows apart
+    int count;
+};
+
 template <int TILE_M>
-__host__ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t) {
+__host__ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t, const RowTiles rt) {
+    const int m_blocks = rt.list != nullptr ? rt.count : p.m_blocks;
     Tile tl;
     tl.skip = false;
     tl.b_row = 0;
@@ -137,21 +150,28 @@ __host__ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t) {
     tl.k_blocks = (p.K + BK - 1) / BK;
     int grp = 0;
     if (p.k_begin != nullptr) {  // grouped-K: one dense [M,N] problem per group
-        int per = p.m_blocks * p.n_blocks;
+        int per = m_blocks * p.n_blocks;
         grp = t / per;
         t -= grp * per;
     }
     int per_group = p.group_m * p.n_blocks;
     int g = t / per_group;
     int first_m = g * p.group_m;
-    int gsz = p.m_blocks - first_m < p.group_m ? p.m_blocks - first_m : p.group_m;
+    int gsz = m_blocks - first_m < p.group_m ? m_blocks - first_m : p.group_m;
     int r = t - g * per_group;
     int mb = first_m + r % gsz;
     int nb = r / gsz;
     mb += p.m_rot;
-    if (mb >= p.m_blocks)
-        mb -= p.m_blocks;
+    if (mb >= m_blocks)
+        mb -= m_blocks;
     tl.m0 = mb * TILE_M;
+    tl.rows = p.M - tl.m0 < TILE_M ? p.M - tl.m0 : TILE_M;
+    if (rt.list != nullptr) {
+        const int entry = rt.list[mb];
+        mb = entry & 0x3fff;
+        tl.m0 = mb * BM;
+        tl.rows = ((entry >> 14) + 1) * BM;
+    }
     tl.n0 = nb * p.n_tile_stride;
     tl.d_row0 = tl.m0;
     if (p.k_begin != nullptr) {
@@ -332,7 +352,7 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, 
     const int m = tl.m0 + row_in_tile;
     const bool row_ok = m < p.M;
     const long drow = tl.d_row0 + row_in_tile;
-    const bool rows_in = tl.m0 + row_base < p.M;  // warp-uniform: some of the 32 rows exist
+    const bool rows_in = row_base < tl.rows;  // warp-uniform: some of the 32 rows exist
     const int box_row = static_cast<int>(tl.d_row0 + row_base);
     if (EPI == EPI_SWIGLU) {
         // columns [0,128) = gate, [128,256) = up of output columns n0..n0+127
@@ -532,6 +552,34 @@ __device__ __forceinline__ void all_gather_warps(const FuseArgs& f, uint64_t lim
     }
 }
 
+// Fills the row-tile list of a grouped problem (one warp; R blocks per tile at most).
+template <int R>
+__device__ __forceinline__ void build_row_tiles(const KParams& p, uint16_t* list, int* count, int lane) {
+    const int blocks = (p.M + BM - 1) / BM;
+    int n = 0, prev = -2, prev_pos = 0;  // group of the block before this batch, its place in its run
+    for (int b0 = 0; b0 < blocks; b0 += 32) {
+        const int b = b0 + lane;
+        const int g = b < blocks ? p.m_block_group[b] : -1;
+        const int left = __shfl_up_sync(0xffffffffu, g, 1);
+        const bool starts = g != (lane == 0 ? prev : left);
+        const uint32_t runs = __ballot_sync(0xffffffffu, starts) & (0xffffffffu >> (31 - lane));
+        const int pos = runs != 0 ? lane - (31 - __clz(runs)) : prev_pos + 1 + lane;
+        const bool first = g >= 0 && pos % R == 0;
+        const uint32_t firsts = __ballot_sync(0xffffffffu, first);
+        if (first) {
+            int more = 0;
+            while (more + 1 < R && b + more + 1 < blocks && p.m_block_group[b + more + 1] == g)
+                ++more;
+            list[n + __popc(firsts & ((1u << lane) - 1u))] = static_cast<uint16_t>(b | (more << 14));
+        }
+        n += __popc(firsts);
+        prev = __shfl_sync(0xffffffffu, g, 31);
+        prev_pos = __shfl_sync(0xffffffffu, pos, 31);
+    }
+    if (lane == 0)
+        *count = n;
+}
+
 template <int MODE, bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
         gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -572,6 +620,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     const uint32_t tfull0 = smem_u32(bars + 2 * STAGES);
     const uint32_t tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
+    constexpr bool ROW_TILES = C::TILE_M > BM && (EPI == EPI_STORE || EPI == EPI_SWIGLU || EPI == EPI_DSWIGLU);
+    uint16_t* row_list = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + BAR_BYTES);
+    int* row_count = reinterpret_cast<int*>(tmem_slot + 8);
+    RowTiles rt{nullptr, 0};
+    if (ROW_TILES && p.m_block_group != nullptr) {
+        if (warp == 2)
+            build_row_tiles<C::TILE_M / BM>(p, row_list, row_count, lane);
+        rt.list = row_list;
+    }
+
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         *split_state = 0;
@@ -607,6 +665,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (rt.list != nullptr)
+        rt.count = *row_count;
+    const int num_tiles = rt.list != nullptr ? rt.count * p.n_blocks : p.num_tiles;
 
     WaitCtx wc{abort_flag, p.wait_limit_ns};
 
@@ -616,8 +677,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             int s = 0;
             uint32_t ph = 0;
             bool alive = true, ready = false;
-            for (int t = worker; t < p.num_tiles && alive; t += workers) {
-                Tile tl = decode_tile<C::TILE_M>(p, t);
+            for (int t = worker; t < num_tiles && alive; t += workers) {
+                Tile tl = decode_tile<C::TILE_M>(p, t, rt);
                 if (tl.skip || tl.k_blocks == 0)
                     continue;
                 // this CTA's rows of A: 128 of each 256-row sub-tile
@@ -685,10 +746,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                     } else {
                         // both CTAs' bytes complete on the leader's barrier
                         const uint32_t fb = mapa_u32(full0 + 8 * s, 0);
+                        const int subs = MSUB > 1 && tl.rows <= 256 ? 1 : MSUB;  // sub-tiles that hold any row
                         if (crank == 0)
-                            mbar_expect_tx(full0 + 8 * s, 2 * C::STAGE_BYTES);
+                            mbar_expect_tx(full0 + 8 * s, 2 * (subs * A_SUB_BYTES + C::B_STAGE_BYTES));
 #pragma unroll
                         for (int sub = 0; sub < MSUB; ++sub) {
+                            if (sub >= subs)
+                                break;
                             const uint32_t sas = sa + sub * A_SUB_BYTES;
                             const int ms = m0 + sub * 256;
                             if (!A_MN) {
@@ -725,8 +789,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             int acc = 0;
             uint32_t acc_ph = 0;
             bool alive = true, ready = false;
-            for (int t = worker; t < p.num_tiles && alive; t += workers) {
-                Tile tl = decode_tile<C::TILE_M>(p, t);
+            for (int t = worker; t < num_tiles && alive; t += workers) {
+                Tile tl = decode_tile<C::TILE_M>(p, t, rt);
                 if (tl.skip || tl.k_blocks == 0)
                     continue;
                 if (MSUB == 1) {
@@ -754,6 +818,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                             }
                             tc_fence_after();
                         }
+                        if (MSUB > 1 && sub > 0 && tl.rows <= 256)
+                            break;  // the second sub-tile holds no rows
                         const uint32_t d_tmem = tmem_base + (MSUB > 1 ? sub : acc) * BN;
                         const uint32_t sa = smem_u32(smem_a + s * A_STAGE_BYTES + sub * A_SUB_BYTES);
 #pragma unroll
@@ -848,8 +914,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             int acc = 0;
             uint32_t acc_ph = 0;
             int ordinal = 0;
-            for (int t = worker; t < p.num_tiles; t += workers) {
-                Tile tl = decode_tile<C::TILE_M>(p, t);
+            for (int t = worker; t < num_tiles; t += workers) {
+                Tile tl = decode_tile<C::TILE_M>(p, t, rt);
                 if (tl.skip)
                     continue;
                 const bool zero_tile = tl.k_blocks == 0;
@@ -904,7 +970,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                     const int sub_row = sub * 256 + static_cast<int>(crank) * BM;  // this CTA's rows of the sub-tile
                     const uint32_t t_addr =
                             tmem_base + (MSUB > 1 ? sub : acc) * BN + (static_cast<uint32_t>(q * 32) << 16);
-                    epilogue_tile<EPI>(p, tl, t_addr, sub_row + q * 32, lane, zero_tile, stage_warp, out, abort_flag);
+                    if (sub_row + q * 32 < tl.rows)
+                        epilogue_tile<EPI>(p, tl, t_addr, sub_row + q * 32, lane, zero_tile, stage_warp, out, abort_flag);
                     if (!zero_tile) {
                         tc_fence_before();
                         __syncwarp();
@@ -1122,15 +1189,47 @@ Plan plan_tiles(const GemmArgs& a, KParams* kpp, int sms) {
     }();
     const int variant = a.variant != 0 ? a.variant : env_variant;
     Plan pl;
-    pl.pair = !grouped_m && variant != 1 && a.M > 128;
+    pl.pair = variant != 1 && a.M > 128;
+    if (grouped_m) {
+        // Tiles of two 128-row blocks of one group (row-tile list) once a group has several blocks; the
+        // capacity M / groups is an upper bound of a group's rows.  8 experts of 4096 rows, 4096 ->
+        // 14336: SwiGLU product 6.64 ms on the 128-row tile, 5.59 on the 256-row tile; 16 experts of 250
+        // rows, down product: 0.66 and 0.48 ms; 16 of 31 rows: 0.31 and 0.37 ms.  The 512-row tile is
+        // no better than the 256-row one and loses up to a quarter on short groups.
+        const bool can = (a.epilogue == EPI_STORE || a.epilogue == EPI_SWIGLU || a.epilogue == EPI_DSWIGLU) &&
+                         (a.M + BM - 1) / BM <= MAX_ROW_TILES && a.m_rot == 0;
+        const long rows = a.M / (a.grouped.groups > 0 ? a.grouped.groups : 1);
+        pl.pair = pl.pair && can && (variant != 0 || rows >= 384);
+    }
     pl.wide = pl.pair && variant == 3;
-    if (pl.pair && variant == 0 && !grouped_k) {
-        const long tiles_wide = static_cast<long>((a.M + 511) / 512) *
-                                ((a.N + (a.epilogue == EPI_SWIGLU ? 127 : 255)) / (a.epilogue == EPI_SWIGLU ? 128 : 256));
+    if (pl.pair && variant == 0 && !grouped_m && a.epilogue != EPI_DSWIGLU) {
         // (the dSwiGLU epilogue reads and writes four values per accumulator element; it needs
         // the next tile's main loop to hide behind: 12.9-13.2 ms on the pair tile against
         // 13.3-14.0 ms on the wide one for 32768 x 28672 x 8192)
-        pl.wide = a.M >= 1024 && a.K >= 3072 && tiles_wide >= 2L * (sms / 2) && a.epilogue != EPI_DSWIGLU;
+        const bool swiglu = a.epilogue == EPI_SWIGLU;
+        const int col = swiglu ? 128 : 256;
+        const long per = (a.N + col - 1) / col, workers = sms / 2 > 0 ? sms / 2 : 1, kb = (a.K + BK - 1) / BK;
+        const long tiles_wide = (a.M + 511) / 512 * per, tiles_pair = (a.M + 255) / 256 * per;
+        if (a.a_ready != nullptr || a.fuse.ag_dst != nullptr || a.fuse.rs_out != nullptr || a.epilogue == EPI_PUSH) {
+            pl.wide = a.M >= 1024 && a.K >= 3072 && tiles_wide >= 2 * workers;
+        } else if (grouped_k) {
+            // ranges so short that writing the result is the work: eight epilogue warps against four
+            // (16 experts of 31 rows, 4096 x 14336 gradients: 0.63 -> 0.52 ms)
+            pl.wide = a.M % 512 == 0 && a.grouped.groups > 0 && a.K / a.grouped.groups < 512;
+        } else if (a.M > 256) {
+            // The wide tile reads less per FLOP but has half as many tiles to fill the waves with and hides
+            // only half of its epilogue.  Estimated times in microseconds, fitted to 1024 x 8192 x 1024
+            // (17.2 on the pair tile, 18.2 on the wide one), 4096 x 4096 x 256 (18.3, 17.0), 4096 x 4096 x
+            // 16384 (376, 361), 14336 x 2048 x 4096 (162, 191), SwiGLU 4096 x 7168 x 2048 (166, 202).
+            const double waves_wide = static_cast<double>((tiles_wide + workers - 1) / workers);
+            const double waves_pair = static_cast<double>((tiles_pair + workers - 1) / workers);
+            const double step = swiglu ? 0.385 : 0.345, tail = swiglu ? 6.0 : 1.2;
+            const double tile_pair = step * kb > 2.9 ? step * kb : 2.9, tile_wide = 0.67 * kb + tail > 4.5 ? 0.67 * kb + tail : 4.5;
+            // Products of many waves run at the power limit, where what the tile does not read counts too:
+            // with the pair tile for K = 3584 the step of 8192/3584 on 32768 tokens was 2 % slower.
+            const double power = kb >= 48 && waves_pair > 8 ? 0.9 : kb >= 64 ? 0.97 : 1.0;
+            pl.wide = (8.0 + waves_wide * tile_wide) * power < 6.6 + waves_pair * tile_pair;
+        }
     }
     // GEMM -> reduce_scatter waits, in the tiles of the rows it owns, for the other ranks' tiles of
     // the same rows.  That cannot deadlock as long as those tiles come strictly earlier in the
@@ -1178,7 +1277,8 @@ int tile_schedule(const GemmArgs& a, int sms, int* tiles, int max_tiles) {
     KParams kp{};
     const Plan pl = plan_tiles(a, &kp, sms);
     for (int t = 0; t < kp.num_tiles && t < max_tiles; ++t) {
-        const Tile tl = pl.wide ? decode_tile<512>(kp, t) : pl.pair ? decode_tile<256>(kp, t) : decode_tile<128>(kp, t);
+        const RowTiles rt{nullptr, 0};
+        const Tile tl = pl.wide ? decode_tile<512>(kp, t, rt) : pl.pair ? decode_tile<256>(kp, t, rt) : decode_tile<128>(kp, t, rt);
         tiles[4 * t + 0] = tl.m0;
         tiles[4 * t + 1] = tl.n0;
         tiles[4 * t + 2] = pl.tile_m;
