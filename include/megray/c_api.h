@@ -27,7 +27,9 @@ typedef struct {
     int aux_off;
     int m_rot;
     int sm_limit;
-    int variant;     /* 0 automatic, 1 single-CTA 128x256 tile, 2 CTA-pair 256x256 tile, 3 CTA-pair 512x256 tile */
+    int variant;     /* 0 automatic, 1 single-CTA 128x256 tile, 2 CTA-pair 256x256 tile, 3 CTA-pair 512x256 tile,
+                        columns + splits (64, 128 or 256, plus 1, 2, 4 or 8): 128-row tile of that many columns whose
+                        K loop a cluster of that many CTAs shares */
     const uint32_t* a_ready;
     int rows_per_flag;
     uint32_t a_ready_target;

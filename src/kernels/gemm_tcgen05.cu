@@ -35,6 +35,7 @@
 #include <map>
 #include <mutex>
 
+#include "gemm_split.cuh"
 #include "launch_count.h"
 
 namespace mgk {
@@ -1269,6 +1270,73 @@ Plan plan_tiles(const GemmArgs& a, KParams* kpp, int sms) {
     kp.k_end = a.grouped.k_end;
     return pl;
 }
+
+// Whether a problem goes to the small-tile / cluster split-K kernel, and with which tile.
+//
+// Only problems whose 128 x 256 tiles fit the chip in one wave are considered: there the persistent
+// kernel leaves SMs idle or, with few k-steps, is all prologue and epilogue (296 x 328 x 456: 9.6 ->
+// 6.1 us; 128 x 8192 x 28672: 176 -> 83 us; 1024 x 1024 x 4096: 24.6 -> 13.3 us); with more tiles the
+// CTA-pair kernel moves less data per FLOP and wins.  Within them a plan is chosen by an estimate
+// whose constants (microseconds) were fitted to 90 shapes from 128 x 256 x 256 to 4096 x 1024 x 16384:
+// launch 1.2 and 3.0 for each wave of CTAs; a k-step by tile width with up to half of the SMs in use, with all of them, and with
+// two CTAs on each; the epilogue and the exchange of the partials by tile width.
+SplitPlan plan_split(const GemmArgs& a, int sms) {
+    const bool swiglu = a.epilogue == EPI_SWIGLU;
+    const bool grouped_m = a.grouped.m_block_group != nullptr, grouped_k = a.grouped.k_begin != nullptr;
+    if (a.variant >= 64)  // asked for by name: variant = columns + splits
+        return SplitPlan{a.variant & ~63, a.variant & 63};
+    static const bool env_variant = getenv("MEGRAY_GEMM_VARIANT") != nullptr;
+    if (a.variant != 0 || env_variant)
+        return SplitPlan{0, 0};
+    const int groups = grouped_k && a.grouped.groups > 0 ? a.grouped.groups : 1;
+    long m_blocks = (a.M + BM - 1) / BM;
+    if (grouped_m)  // the row capacity holds about a quarter more blocks than are in use
+        m_blocks = m_blocks - m_blocks / 5;
+    const long kb = ((a.K + BK - 1) / BK + groups - 1) / groups;
+    const long tiles256 = m_blocks * ((a.N + (swiglu ? 127 : 255)) / (swiglu ? 128 : 256)) * groups;
+    const bool one_row = !grouped_m && !grouped_k && a.M <= BM;
+    if (!one_row && tiles256 > sms + sms / 12)
+        return SplitPlan{0, 0};
+    // what the persistent kernel adds to its main loop, and this one per 64 columns, by epilogue
+    const double extra_pair = a.epilogue == EPI_DSWIGLU ? 9.5 : a.epilogue == EPI_ACCUM ? 4.2 : a.epilogue == EPI_STORE ? 0.0 : 1.6;
+    const double extra = a.epilogue == EPI_DSWIGLU ? 2.0 : a.epilogue == EPI_ACCUM ? 1.0 : swiglu ? 0.5 : a.epilogue == EPI_STORE ? 0.0 : 0.3;
+    double best_t = one_row ? 1e30 : 0.97 * (6.6 + 0.32 * kb + extra_pair);
+    SplitPlan best{0, 0};
+    for (int i = 0; i < 3; ++i) {
+        static const double step1[3] = {0.14, 0.15, 0.28}, stepn[3] = {0.16, 0.20, 0.32}, step2[3] = {0.31, 0.445, 0.75};
+        static const double tail1[3] = {0.0, 0.7, 1.9}, tailS[3] = {1.5, 2.8, 5.7};
+        const int bn = 64 << i, shift = 6 + i - (swiglu ? 1 : 0);
+        const long tiles = m_blocks * ((a.N + (1 << shift) - 1) >> shift) * groups;
+        for (int lg = 0; lg < 4; ++lg) {
+            const int sp = 1 << lg;
+            const SplitPlan plan{bn, sp};
+            const long ctas = tiles << lg;
+            // 256 columns leave no room for a second CTA beside the exchange buffer
+            const int per_sm = ctas <= sms || (bn == 256 && sp > 1) ? 1 : 2;
+            if (sp > 1 && (ctas > static_cast<long>(sms) * per_sm || kb >> lg < 2))
+                break;
+            if (sp == 8 && ctas > (per_sm == 1 ? 96 : 256))  // clusters of 8 do not pack every SM
+                continue;
+            if (!one_row && bn == 256 && sp == 1 && kb > 128)  // the pair tile hides its epilogue as well
+                continue;
+            const long waves = ctas <= static_cast<long>(sms) * per_sm ? 1 : (ctas - 1) / (sms * per_sm) + 1;
+            double tail = (sp == 1 ? tail1[i] : tailS[i]) + extra * (1 << i) / sp;
+            if (per_sm == 2)
+                tail *= sp == 1 ? 1.5 : 2.0;
+            const double step = per_sm == 2 ? step2[i] : ctas <= sms / 2 ? step1[i] : stepn[i];
+            double t = 1.2 + waves * (3.0 + ((kb + sp - 1) >> lg) * step + tail);
+            if (one_row) {  // bound by reading B once it is large
+                const double read = 2.0 * a.K * (a.M + static_cast<double>(a.N) * (swiglu ? 2 : 1)) / 6.2e6 + 4.0;
+                t = (t > read ? t : read) + 0.1 * t;
+            }
+            if (t < best_t && split_accepts(a, plan)) {
+                best_t = t;
+                best = plan;
+            }
+        }
+    }
+    return best;
+}
 }  // namespace
 
 int tile_schedule(const GemmArgs& a, int sms, int* tiles, int max_tiles) {
@@ -1298,7 +1366,8 @@ cudaError_t launch_gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
     const bool grouped_m = a.grouped.m_block_group != nullptr;
     const bool grouped_k = a.grouped.k_begin != nullptr;
     KParams kp{};
-    const Plan pl = plan_tiles(a, &kp, sm_count());
+    const int sms = sm_count();
+    const Plan pl = plan_tiles(a, &kp, sms);
     const bool pair = pl.pair, wide = pl.wide;
     const int tile_m = pl.tile_m;
     kp.D = static_cast<__nv_bfloat16*>(a.D);
@@ -1329,6 +1398,9 @@ cudaError_t launch_gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
         return cudaErrorInvalidValue;
     if (a.a_ready != nullptr && (kp.rows_per_flag % BM))
         return cudaErrorInvalidValue;
+
+    if (const SplitPlan sp = plan_split(a, sms); sp.bn != 0)
+        return launch_gemm_split(a, sp, sms, stream);
 
     // Extents the tensor maps cover.  Grouped problems stack the groups along the
     // outer dimension of B.
