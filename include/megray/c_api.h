@@ -182,6 +182,41 @@ int megray_add_rmsnorm_bf16(const void* x, const void* y, void* x_out, void* n_o
 int megray_rmsnorm_bwd_bf16(const void* dn, const void* n, const float* inv_rms, const void* dres,
                             void* dx, int rows, int cols, void* stream);
 
+/* ---- one pass of the single-GPU models -----------------------------------------------------------
+ * The launches of megray_b200/models (tp_mlp.py, moe.py without a communicator) as one call each.
+ * All matrices are contiguous bf16, row-major; nothing is kept between calls. */
+typedef struct {
+    int splits;          /* K ranges of a weight-gradient product; <= 1 = unsplit */
+    const int* k_begin;  /* device arrays of `splits` entries */
+    const int* k_end;
+} megray_k_split;
+typedef struct {
+    void *w_gu, *w_down;  /* [2 ffn, d_model], [d_model, ffn] */
+    void *g_gu, *g_down;  /* their gradients */
+    void *xg, *gu, *h;    /* kept for backward: [tokens, d_model], [tokens, 2 ffn], [tokens, ffn] */
+    float* inv_rms;       /* [tokens] */
+} megray_mlp_layer;
+typedef struct {
+    int layers, tokens, d_model, ffn;
+    const megray_mlp_layer* layer;
+    void *xs[2], *y, *dgu, *dn, *dres[2];
+    void* wgrad_ws;       /* float32 partial products of the split weight gradients */
+    megray_k_split split_down, split_gu;
+    int* error_flag;
+} megray_mlp_args;
+int megray_mlp_forward(const megray_mlp_args* a, const void* x, void* stream);    /* result: xs[(layers - 1) & 1] */
+int megray_mlp_backward(const megray_mlp_args* a, const void* dy, void* stream);  /* result: dres[0] */
+typedef struct {
+    int tokens, experts, hidden, ffn, capacity;
+    void *w_gu, *w_down, *g_gu, *g_down;
+    void *x_perm, *y_perm, *dy_perm, *dx_perm, *gu, *h, *dgu, *out, *dx;
+    int *idx, *pos, *counts, *cursor, *send_base, *seg_begin, *seg_end, *seg_rows, *block_group, *total;
+    float *w, *dw, *dlogits;
+    int* error_flag;
+} megray_moe_args;
+int megray_moe_forward(const megray_moe_args* a, const void* x, const float* logits, void* stream);  /* result: out */
+int megray_moe_backward(const megray_moe_args* a, const void* dout, void* stream);                   /* results: dx, dlogits */
+
 /* Kernels launched by this library since it was loaded (all modules). */
 uint64_t megray_launch_count(void);
 

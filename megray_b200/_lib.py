@@ -51,6 +51,37 @@ class GemmArgs(C.Structure):
     ]
 
 
+class KSplit(C.Structure):
+    """Mirror of ``megray_k_split``."""
+
+    _fields_ = [("splits", C.c_int), ("k_begin", C.c_void_p), ("k_end", C.c_void_p)]
+
+
+class MLPLayer(C.Structure):
+    """Mirror of ``megray_mlp_layer``."""
+
+    _fields_ = [(n, C.c_void_p) for n in ("w_gu", "w_down", "g_gu", "g_down", "xg", "gu", "h", "inv_rms")]
+
+
+class MLPArgs(C.Structure):
+    """Mirror of ``megray_mlp_args``."""
+
+    _fields_ = ([(n, C.c_int) for n in ("layers", "tokens", "d_model", "ffn")] +
+                [("layer", C.POINTER(MLPLayer)), ("xs", C.c_void_p * 2), ("y", C.c_void_p), ("dgu", C.c_void_p),
+                 ("dn", C.c_void_p), ("dres", C.c_void_p * 2), ("wgrad_ws", C.c_void_p), ("split_down", KSplit),
+                 ("split_gu", KSplit), ("error_flag", C.c_void_p)])
+
+
+class MoEArgs(C.Structure):
+    """Mirror of ``megray_moe_args``."""
+
+    _fields_ = ([(n, C.c_int) for n in ("tokens", "experts", "hidden", "ffn", "capacity")] +
+                [(n, C.c_void_p) for n in
+                 ("w_gu", "w_down", "g_gu", "g_down", "x_perm", "y_perm", "dy_perm", "dx_perm", "gu", "h", "dgu", "out",
+                  "dx", "idx", "pos", "counts", "cursor", "send_base", "seg_begin", "seg_end", "seg_rows",
+                  "block_group", "total", "w", "dw", "dlogits", "error_flag")])
+
+
 def _declare(lib) -> None:
     """argtypes / restype of the C interface (include/megray/c_api.h)."""
     vp, u32, u64, i32, i64, sz = C.c_void_p, C.c_uint32, C.c_uint64, C.c_int, C.c_int64, C.c_size_t
@@ -133,6 +164,10 @@ def _declare(lib) -> None:
     d("megray_moe_dispatch", i32, vp, i32, i32, vp, vp, vp, vp, vp, vp, P(vp), i32, i32, i32, vp)
     d("megray_moe_combine", i32, vp, i32, i32, vp, vp, vp, P(vp), i32, i32, i32, vp)
     d("megray_moe_combine_dw", i32, vp, i32, i32, vp, vp, P(vp), i32, i32, i32, vp, vp)
+    d("megray_mlp_forward", i32, P(MLPArgs), vp, vp)
+    d("megray_mlp_backward", i32, P(MLPArgs), vp, vp)
+    d("megray_moe_forward", i32, P(MoEArgs), vp, vp, vp)
+    d("megray_moe_backward", i32, P(MoEArgs), vp, vp)
     d("megray_dtype_size", sz, i32)
     d("megray_set_log_level", None, i32)
     d("megray_trace_enable", None, C.c_char_p)
@@ -142,6 +177,8 @@ def _declare(lib) -> None:
 def load(build_if_missing: bool = True) -> C.CDLL:
     """Load the native library (building it first when it is absent)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib

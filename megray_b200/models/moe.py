@@ -19,8 +19,12 @@ from dataclasses import dataclass
 
 import torch
 
+from .. import _lib
 from ..ops import EPI_DSWIGLU, EPI_SWIGLU, gemm, mse_loss_grad, sgd_step
+from ..ops.gemm import gemm_error_flag
 from ..parallel.expert_parallel import ExpertParallelOps
+from ..ops._stream import raw_stream
+from ._native import plain
 
 
 @dataclass
@@ -74,9 +78,31 @@ class MoELayer:
         self.x_dev = torch.empty(T, H, **bf)
         self.logits_dev = torch.empty(T, cfg.experts, dtype=torch.float32, device=self.device)
 
+    def _native_args(self):
+        """Argument block of the native passes for this call; None with a communicator, or when a weight
+        or gradient is not the contiguous matrix they take."""
+        ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
+        if self.comm is not None:
+            return None
+        gu, down = (ep.El * 2 * F, H), (ep.El * H, F)
+        p = (plain(self.w_gu, gu), plain(self.w_down, down), plain(self.g_gu, gu), plain(self.g_down, down))
+        if 0 in p:
+            return None
+        rest = (self.x_perm, self.y_perm, self.dy_perm, self.dx_perm, self.gu, self.h, self.dgu, self.out, self.dx,
+                ep.idx, ep.pos, ep.counts, ep.cursor, ep.send_base, ep.seg_begin, ep.seg_end, ep.seg_rows,
+                ep.block_group, ep.total, ep.w, self.dw, self.dlogits, gemm_error_flag(self.out.device))
+        return _lib.MoEArgs(ep.T, ep.E, H, F, ep.capacity, *p, *[t.data_ptr() for t in rest])
+
     # ------------------------------------------------------------------ forward / backward
     def forward(self, x: torch.Tensor, logits: torch.Tensor) -> torch.Tensor:
         ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
+        px, pl = plain(x, (ep.T, H)), plain(logits, (ep.T, ep.E), torch.float32)
+        args = self._native_args() if px and pl else None
+        if args is not None:
+            rc = _lib.load().megray_moe_forward(args, px, pl, raw_stream())
+            if rc != 0:
+                raise RuntimeError(f"megray_moe_forward failed ({rc})")
+            return self.out
         ep.route(logits)
         ep.plan()
         ep.zero_pads(self.x_perm)
@@ -92,6 +118,13 @@ class MoELayer:
     def backward(self, dout: torch.Tensor):
         """Returns (dx, dlogits); fills the expert weight gradients."""
         ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
+        pd = plain(dout, (ep.T, H))
+        args = self._native_args() if pd else None
+        if args is not None:
+            rc = _lib.load().megray_moe_backward(args, pd, raw_stream())
+            if rc != 0:
+                raise RuntimeError(f"megray_moe_backward failed ({rc})")
+            return self.dx, self.dlogits
         ep.combine_dw(dout, self.y_perm, self.dw)
         ep.zero_pads(self.dy_perm)
         ep.dispatch(dout, self.dy_perm, weights=True, first=False)

@@ -29,8 +29,12 @@ from typing import List, Optional
 
 import torch
 
+from .. import _lib
 from ..ops import (EPI_DSWIGLU, EPI_SWIGLU, add_rmsnorm, gemm, gemm_split_k, mse_loss_grad, pick_split_k,
                    rmsnorm_bwd, sgd_step)
+from ..ops.gemm import gemm_error_flag, split_ranges
+from ..ops._stream import raw_stream
+from ._native import plain
 
 
 @dataclass
@@ -113,10 +117,38 @@ class TPMLPStack:
         """This rank's rows of an all-token buffer."""
         return full[self.rank * self.Ts:(self.rank + 1) * self.Ts]
 
+    def _native_args(self):
+        """Argument block of the native passes for this call; None on several ranks, or when a weight
+        or gradient is not the contiguous matrix they take."""
+        if self.tp is not None or self.n != 1:
+            return None
+        T, d, f, L = self.Ts, self.cfg.d_model, self.cfg.ffn, len(self.layers)
+        gu, down = (2 * f, d), (d, f)
+        layers = (_lib.MLPLayer * L)()
+        for l, w in enumerate(self.layers):
+            p = (plain(w.w_gu, gu), plain(w.w_down, down), plain(w.g_gu, gu), plain(w.g_down, down))
+            if 0 in p:
+                return None
+            layers[l] = _lib.MLPLayer(*p, self.xg[l].data_ptr(), self.gu[l].data_ptr(), self.h[l].data_ptr(),
+                                      self.inv_rms[l].data_ptr())
+        a = _lib.MLPArgs(L, T, d, f, layers)
+        a.xs[0], a.xs[1] = self.xs[0].data_ptr(), self.xs[1].data_ptr()
+        a.dres[0], a.dres[1] = self.dres[0].data_ptr(), self.dres[1].data_ptr()
+        a.y, a.dgu, a.dn = self.y.data_ptr(), self.dgu.data_ptr(), self.dn.data_ptr()
+        a.error_flag = gemm_error_flag(self.y.device).data_ptr()
+        return a
+
     # ------------------------------------------------------------------ forward / backward
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """x: this rank's [T/n, d] token shard (bf16).  Returns the [T/n, d] output shard."""
         L = len(self.layers)
+        px = plain(x, (self.Ts, self.cfg.d_model))
+        args = self._native_args() if px else None
+        if args is not None:
+            rc = _lib.load().megray_mlp_forward(args, px, raw_stream())
+            if rc != 0:
+                raise RuntimeError(f"megray_mlp_forward failed ({rc})")
+            return self.xs[(L - 1) & 1]
         add_rmsnorm(x, None, None, self._shard(self.xg[0]), self.inv_rms[0])
         for l, layer in enumerate(self.layers):
             fl = layer.fl
@@ -140,6 +172,23 @@ class TPMLPStack:
         if self.dy0 is not None and dy is not self.dy0:
             self.dy0.copy_(dy)  # the backward gather reads its source from peers' heaps
             dy = self.dy0
+        pdy = plain(dy, (self.Ts, self.cfg.d_model))
+        args = self._native_args() if pdy else None
+        if args is not None:
+            T, d, f = self.Ts, self.cfg.d_model, self.cfg.ffn
+            need = 0
+            for split, M, N in ((args.split_down, d, f), (args.split_gu, 2 * f, d)):
+                split.splits = s = pick_split_k(M, N, T)
+                if s > 1:
+                    begin, end = split_ranges(dy.device, T, s)
+                    split.k_begin, split.k_end = begin.data_ptr(), end.data_ptr()
+                    need = max(need, s * M * N)
+            if need:
+                args.wgrad_ws = self._partials(need).data_ptr()
+            rc = _lib.load().megray_mlp_backward(args, pdy, raw_stream())
+            if rc != 0:
+                raise RuntimeError(f"megray_mlp_backward failed ({rc})")
+            return self.dres[0]
         dres = dy
         for l in reversed(range(len(self.layers))):
             layer = self.layers[l]
@@ -168,10 +217,14 @@ class TPMLPStack:
         if splits == 1:
             gemm(a_t, b_t, out, a_mn=True, b_mn=True)
             return
-        need = splits * M * N
+        ws = self._partials(splits * M * N)
+        gemm_split_k(a_t, b_t, out, splits, ws.view(splits * M, N), a_mn=True, b_mn=True)
+
+    def _partials(self, need: int) -> torch.Tensor:
+        """Workspace of ``need`` floats for partial products, kept by the model."""
         if self._wgrad_ws is None or self._wgrad_ws.numel() < need:
             self._wgrad_ws = torch.empty(need, dtype=torch.float32, device=self.device)
-        gemm_split_k(a_t, b_t, out, splits, self._wgrad_ws[:need].view(splits * M, N), a_mn=True, b_mn=True)
+        return self._wgrad_ws[:need]
 
     def optimizer_step(self) -> None:
         for layer in self.layers:

@@ -2,15 +2,10 @@
 squared-error loss with its gradient."""
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
 from .. import _lib
-
-
-def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+from ._stream import raw_stream
 
 
 def sgd_step(w: torch.Tensor, g: torch.Tensor, lr: float, momentum_buf: torch.Tensor = None,
@@ -19,7 +14,7 @@ def sgd_step(w: torch.Tensor, g: torch.Tensor, lr: float, momentum_buf: torch.Te
     assert w.dtype == torch.bfloat16 and g.dtype == torch.bfloat16 and w.is_contiguous() and g.is_contiguous()
     mp = momentum_buf.data_ptr() if momentum_buf is not None else None
     rc = _lib.load().megray_sgd_bf16(w.data_ptr(), g.data_ptr(), mp, w.numel(), lr, momentum, weight_decay,
-                                     _stream())
+                                     raw_stream())
     if rc != 0:
         raise RuntimeError(f"megray_sgd_bf16 failed ({rc})")
 
@@ -37,7 +32,7 @@ def mse_loss_grad(y: torch.Tensor, target: torch.Tensor = None, scale: float = N
         dy = torch.empty_like(y)
     tp = target.data_ptr() if target is not None else None
     rc = _lib.load().megray_mse_bf16(y.data_ptr(), tp, dy.data_ptr(), loss.data_ptr(), y.numel(), scale,
-                                     _stream())
+                                     raw_stream())
     if rc != 0:
         raise RuntimeError(f"megray_mse_bf16 failed ({rc})")
     return loss, dy
@@ -51,7 +46,7 @@ def add_rmsnorm(x: torch.Tensor, y: torch.Tensor = None, x_out: torch.Tensor = N
     assert x.dtype == torch.bfloat16 and x.is_contiguous()
     p = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
     rc = _lib.load().megray_add_rmsnorm_bf16(p(x), p(y), p(x_out), p(n_out), p(inv_rms), rows, cols, eps,
-                                             _stream())
+                                             raw_stream())
     if rc != 0:
         raise RuntimeError(f"megray_add_rmsnorm_bf16 failed ({rc})")
 
@@ -61,6 +56,6 @@ def rmsnorm_bwd(dn: torch.Tensor, n: torch.Tensor, inv_rms: torch.Tensor, dres: 
     """dx = dres + inv_rms * (dn - n * mean(dn * n)) per row (dres optional)."""
     rows, cols = dn.shape
     p = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
-    rc = _lib.load().megray_rmsnorm_bwd_bf16(p(dn), p(n), p(inv_rms), p(dres), p(dx), rows, cols, _stream())
+    rc = _lib.load().megray_rmsnorm_bwd_bf16(p(dn), p(n), p(inv_rms), p(dres), p(dx), rows, cols, raw_stream())
     if rc != 0:
         raise RuntimeError(f"megray_rmsnorm_bwd_bf16 failed ({rc})")

@@ -24,6 +24,7 @@ import ctypes as C
 import torch
 
 from .. import _lib
+from ._stream import raw_stream
 
 EPI_STORE, EPI_SWIGLU, EPI_DSWIGLU, EPI_ACCUM, EPI_PUSH, EPI_STORE_ROWS, EPI_STORE_F32 = 0, 1, 2, 3, 4, 5, 6
 
@@ -32,7 +33,10 @@ _err_flags = {}
 
 def gemm_error_flag(device=None) -> torch.Tensor:
     """Per-device int32 word the kernels set when one of their bounded waits ran out."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    if device is None:
+        dev = torch.device("cuda", torch.cuda.current_device())
+    else:
+        dev = device if isinstance(device, torch.device) else torch.device(device)
     key = dev.index
     if key not in _err_flags:
         _err_flags[key] = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -40,9 +44,10 @@ def gemm_error_flag(device=None) -> torch.Tensor:
 
 
 def _check2d(t: torch.Tensor, name: str, dtype=torch.bfloat16) -> None:
-    if t.dtype != dtype or t.dim() != 2 or not t.is_cuda:
+    stride = t.stride()
+    if t.dtype != dtype or len(stride) != 2 or not t.is_cuda:
         raise ValueError(f"{name}: expected a 2-D CUDA {dtype} tensor")
-    if t.stride(1) != 1 or t.stride(0) % 8 != 0 or t.data_ptr() % 16 != 0:
+    if stride[1] != 1 or stride[0] % 8 != 0 or t.data_ptr() % 16 != 0:
         raise ValueError(f"{name}: rows must be contiguous, 16-byte aligned, leading dimension % 8 == 0")
 
 
@@ -73,17 +78,12 @@ def build_gemm_args(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, 
     out_dtype = torch.float32 if epilogue == EPI_STORE_F32 else torch.bfloat16
     if out is None and alloc_out:
         out = torch.empty(out_rows, out_cols, dtype=out_dtype, device=a.device)
-    args = _lib.GemmArgs()
-    args.A, args.B = a.data_ptr(), b.data_ptr()
+    d, ldd = None, out_cols
     if out is not None:
         _check2d(out, "out", out_dtype)
-        args.D, args.ldd = out.data_ptr(), out.stride(0)
-    else:
-        args.ldd = out_cols
-    args.M, args.N, args.K = M, N, K
-    args.lda, args.ldb = a.stride(0), b.stride(0)
-    args.a_mn, args.b_mn, args.epilogue, args.aux_off = int(a_mn), int(b_mn), epilogue, aux_off
-    args.m_rot, args.sm_limit, args.variant = m_rot, sm_limit, variant
+        d, ldd = out.data_ptr(), out.stride(0)
+    args = _lib.GemmArgs(a.data_ptr(), b.data_ptr(), d, None, None, M, N, K, a.stride(0), b.stride(0), ldd, 0, 0,
+                         int(a_mn), int(b_mn), epilogue, aux_off, m_rot, sm_limit, variant)
     if epilogue == EPI_SWIGLU:
         if out2 is None:
             out2 = torch.empty(M, N, dtype=torch.bfloat16, device=a.device)
@@ -112,7 +112,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, **kw) -> to
     the output width (needed for SWIGLU, where the logical N is F while ``b`` has 2F rows, and
     for grouped problems)."""
     args, out, out2 = build_gemm_args(a, b, out, **kw)
-    rc = _lib.load().megray_gemm_bf16(C.byref(args), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    rc = _lib.load().megray_gemm_bf16(args, raw_stream())
     if rc != 0:
         raise RuntimeError(f"megray_gemm_bf16 failed (code {rc}) for M={args.M} N={args.N} K={args.K}")
     return (out, out2) if args.epilogue == EPI_SWIGLU else out
@@ -149,6 +149,20 @@ def pick_split_k(M: int, N: int, K: int, sms: int = 148) -> int:
     return best
 
 
+def split_ranges(device: torch.device, K: int, splits: int):
+    """Device arrays with the first row of each of ``splits`` ranges of K and one past its last."""
+    key = (device.index, K, splits)
+    if key not in _split_ranges:
+        per = -(-(-(-K // 64)) // splits) * 64  # ceil(ceil(K / 64) / splits) * 64
+        begin = [min(K, i * per) for i in range(splits)]
+        end = [min(K, (i + 1) * per) for i in range(splits)]
+        if any(e <= s for s, e in zip(begin, end)):
+            raise ValueError("gemm_split_k: K is too short for this many ranges")
+        _split_ranges[key] = (torch.tensor(begin, dtype=torch.int32, device=device),
+                              torch.tensor(end, dtype=torch.int32, device=device))
+    return _split_ranges[key]
+
+
 def gemm_split_k(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, splits: int, partial: torch.Tensor = None,
                  *, a_mn: bool = False, b_mn: bool = False) -> torch.Tensor:
     """``out = A @ B^T`` computed as ``splits`` partial products over disjoint K ranges (multiples
@@ -161,16 +175,7 @@ def gemm_split_k(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, splits: in
     N = b.shape[1] if b_mn else b.shape[0]
     if splits > 8 or M % 256 or not out.is_contiguous() or out.shape != (M, N):
         raise ValueError("gemm_split_k: at most 8 ranges, M a multiple of 256, contiguous [M, N] output")
-    per = -(-(-(-K // 64)) // splits) * 64  # ceil(ceil(K / 64) / splits) * 64
-    key = (a.device.index, K, splits)
-    if key not in _split_ranges:
-        begin = [min(K, i * per) for i in range(splits)]
-        end = [min(K, (i + 1) * per) for i in range(splits)]
-        if any(e <= s for s, e in zip(begin, end)):
-            raise ValueError("gemm_split_k: K is too short for this many ranges")
-        _split_ranges[key] = (torch.tensor(begin, dtype=torch.int32, device=a.device),
-                              torch.tensor(end, dtype=torch.int32, device=a.device))
-    k_begin, k_end = _split_ranges[key]
+    k_begin, k_end = split_ranges(a.device, K, splits)
     if partial is None:
         partial = torch.empty(splits * M, N, dtype=torch.float32, device=a.device)
     part = partial[: splits * M]
