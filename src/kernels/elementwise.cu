@@ -335,6 +335,9 @@ cudaError_t launch_sgd_bf16(void* w, const void* g, float* momentum, uint64_t n,
         return cudaSuccess;
     if ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(g)) & 15)
         return cudaErrorInvalidValue;
+    // whole groups read and write the momentum in vectors, fewer than 16 elements one by one
+    if (reinterpret_cast<uintptr_t>(momentum) & (n >= 16 ? 15 : 3))
+        return cudaErrorInvalidValue;
     auto* wb = static_cast<__nv_bfloat16*>(w);
     auto* gb = static_cast<const __nv_bfloat16*>(g);
     const bool wide = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(g) |
