@@ -79,25 +79,44 @@ class MoELayer:
         self.logits_dev = torch.empty(T, cfg.experts, dtype=torch.float32, device=self.device)
 
     def _native_args(self):
-        """Argument block of the native passes for this call; None with a communicator, or when a weight
-        or gradient is not the contiguous matrix they take."""
+        """Argument block of the native passes for this call with what both of them use; None with a
+        communicator, or when a weight is not the contiguous matrix they take."""
         ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
         if self.comm is not None:
             return None
-        gu, down = (ep.El * 2 * F, H), (ep.El * H, F)
-        p = (plain(self.w_gu, gu), plain(self.w_down, down), plain(self.g_gu, gu), plain(self.g_down, down))
+        a = _lib.MoEArgs(ep.T, ep.E, H, F, ep.capacity)
+        a.w_gu, a.w_down = p = plain(self.w_gu, (ep.El * 2 * F, H)), plain(self.w_down, (ep.El * H, F))
         if 0 in p:
             return None
-        rest = (self.x_perm, self.y_perm, self.dy_perm, self.dx_perm, self.gu, self.h, self.dgu, self.out, self.dx,
-                ep.idx, ep.pos, ep.counts, ep.cursor, ep.send_base, ep.seg_begin, ep.seg_end, ep.seg_rows,
-                ep.block_group, ep.total, ep.w, self.dw, self.dlogits, gemm_error_flag(self.out.device))
-        return _lib.MoEArgs(ep.T, ep.E, H, F, ep.capacity, *p, *[t.data_ptr() for t in rest])
+        for name in ("x_perm", "y_perm", "gu", "h"):
+            setattr(a, name, getattr(self, name).data_ptr())
+        for name in ("idx", "pos", "cursor", "send_base", "seg_begin", "seg_end", "seg_rows", "block_group", "w"):
+            setattr(a, name, getattr(ep, name).data_ptr())
+        a.error_flag = gemm_error_flag(self.h.device).data_ptr()
+        return a
+
+    def _native_forward_args(self):
+        a = self._native_args()
+        if a is not None:
+            a.out, a.counts, a.total = self.out.data_ptr(), self.ep.counts.data_ptr(), self.ep.total.data_ptr()
+        return a
+
+    def _native_backward_args(self):
+        a, ep, F, H = self._native_args(), self.ep, self.cfg.ffn, self.cfg.hidden
+        if a is None:
+            return None
+        a.g_gu, a.g_down = p = plain(self.g_gu, (ep.El * 2 * F, H)), plain(self.g_down, (ep.El * H, F))
+        if 0 in p:
+            return None
+        for name in ("dy_perm", "dx_perm", "dgu", "dx", "dw", "dlogits"):
+            setattr(a, name, getattr(self, name).data_ptr())
+        return a
 
     # ------------------------------------------------------------------ forward / backward
     def forward(self, x: torch.Tensor, logits: torch.Tensor) -> torch.Tensor:
         ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
         px, pl = plain(x, (ep.T, H)), plain(logits, (ep.T, ep.E), torch.float32)
-        args = self._native_args() if px and pl else None
+        args = self._native_forward_args() if px and pl else None
         if args is not None:
             rc = _lib.load().megray_moe_forward(args, px, pl, raw_stream())
             if rc != 0:
@@ -119,7 +138,7 @@ class MoELayer:
         """Returns (dx, dlogits); fills the expert weight gradients."""
         ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
         pd = plain(dout, (ep.T, H))
-        args = self._native_args() if pd else None
+        args = self._native_backward_args() if pd else None
         if args is not None:
             rc = _lib.load().megray_moe_backward(args, pd, raw_stream())
             if rc != 0:

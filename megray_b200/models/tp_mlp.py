@@ -118,24 +118,50 @@ class TPMLPStack:
         return full[self.rank * self.Ts:(self.rank + 1) * self.Ts]
 
     def _native_args(self):
-        """Argument block of the native passes for this call; None on several ranks, or when a weight
-        or gradient is not the contiguous matrix they take."""
+        """Argument block of the native passes for this call with what both of them use; None on several
+        ranks, or when a weight is not the contiguous matrix they take."""
         if self.tp is not None or self.n != 1:
             return None
         T, d, f, L = self.Ts, self.cfg.d_model, self.cfg.ffn, len(self.layers)
-        gu, down = (2 * f, d), (d, f)
         layers = (_lib.MLPLayer * L)()
         for l, w in enumerate(self.layers):
-            p = (plain(w.w_gu, gu), plain(w.w_down, down), plain(w.g_gu, gu), plain(w.g_down, down))
+            p = (plain(w.w_gu, (2 * f, d)), plain(w.w_down, (d, f)))
             if 0 in p:
                 return None
-            layers[l] = _lib.MLPLayer(*p, self.xg[l].data_ptr(), self.gu[l].data_ptr(), self.h[l].data_ptr(),
-                                      self.inv_rms[l].data_ptr())
+            layers[l] = _lib.MLPLayer(*p, None, None, self.xg[l].data_ptr(), self.gu[l].data_ptr(),
+                                      self.h[l].data_ptr(), self.inv_rms[l].data_ptr())
         a = _lib.MLPArgs(L, T, d, f, layers)
-        a.xs[0], a.xs[1] = self.xs[0].data_ptr(), self.xs[1].data_ptr()
+        a.error_flag = gemm_error_flag(self.h[0].device).data_ptr()
+        return a
+
+    def _native_forward_args(self):
+        a = self._native_args()
+        if a is not None:
+            a.y = self.y.data_ptr()
+            a.xs[0], a.xs[1] = self.xs[0].data_ptr(), self.xs[1].data_ptr()
+        return a
+
+    def _native_backward_args(self):
+        a = self._native_args()
+        if a is None:
+            return None
+        T, d, f = self.Ts, self.cfg.d_model, self.cfg.ffn
+        for l, w in enumerate(self.layers):
+            p = (plain(w.g_gu, (2 * f, d)), plain(w.g_down, (d, f)))
+            if 0 in p:
+                return None
+            a.layer[l].g_gu, a.layer[l].g_down = p
+        a.dgu, a.dn = self.dgu.data_ptr(), self.dn.data_ptr()
         a.dres[0], a.dres[1] = self.dres[0].data_ptr(), self.dres[1].data_ptr()
-        a.y, a.dgu, a.dn = self.y.data_ptr(), self.dgu.data_ptr(), self.dn.data_ptr()
-        a.error_flag = gemm_error_flag(self.y.device).data_ptr()
+        need = 0
+        for split, M, N in ((a.split_down, d, f), (a.split_gu, 2 * f, d)):
+            split.splits = s = pick_split_k(M, N, T)
+            if s > 1:
+                begin, end = split_ranges(self.dgu.device, T, s)
+                split.k_begin, split.k_end = begin.data_ptr(), end.data_ptr()
+                need = max(need, s * M * N)
+        if need:
+            a.wgrad_ws = self._partials(need).data_ptr()
         return a
 
     # ------------------------------------------------------------------ forward / backward
@@ -143,7 +169,7 @@ class TPMLPStack:
         """x: this rank's [T/n, d] token shard (bf16).  Returns the [T/n, d] output shard."""
         L = len(self.layers)
         px = plain(x, (self.Ts, self.cfg.d_model))
-        args = self._native_args() if px else None
+        args = self._native_forward_args() if px else None
         if args is not None:
             rc = _lib.load().megray_mlp_forward(args, px, raw_stream())
             if rc != 0:
@@ -173,18 +199,8 @@ class TPMLPStack:
             self.dy0.copy_(dy)  # the backward gather reads its source from peers' heaps
             dy = self.dy0
         pdy = plain(dy, (self.Ts, self.cfg.d_model))
-        args = self._native_args() if pdy else None
+        args = self._native_backward_args() if pdy else None
         if args is not None:
-            T, d, f = self.Ts, self.cfg.d_model, self.cfg.ffn
-            need = 0
-            for split, M, N in ((args.split_down, d, f), (args.split_gu, 2 * f, d)):
-                split.splits = s = pick_split_k(M, N, T)
-                if s > 1:
-                    begin, end = split_ranges(dy.device, T, s)
-                    split.k_begin, split.k_end = begin.data_ptr(), end.data_ptr()
-                    need = max(need, s * M * N)
-            if need:
-                args.wgrad_ws = self._partials(need).data_ptr()
             rc = _lib.load().megray_mlp_backward(args, pdy, raw_stream())
             if rc != 0:
                 raise RuntimeError(f"megray_mlp_backward failed ({rc})")
