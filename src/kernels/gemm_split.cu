@@ -45,9 +45,7 @@ constexpr int min_stages(int bnt, bool split) {
 
 struct SParams {
     int M, N, K;
-    int m_blocks, n_blocks;
-    int group_m;
-    int n_tile_stride;  // BNT, or BNT / 2 for the SwiGLU pairing
+    SplitRaster raster;
     int stages;
     const __nv_bfloat16* D;  // EPI_ACCUM reads it
     long ldd;
@@ -204,17 +202,14 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 2)
     int t = static_cast<int>(blockIdx.x) / splits;
     int grp = 0;
     if (p.k_begin != nullptr) {
-        const int per = p.m_blocks * p.n_blocks;
+        const int per = p.raster.m_blocks * p.raster.n_blocks;
         grp = t / per;
         t -= grp * per;
     }
-    const int per_group = p.group_m * p.n_blocks;
-    const int g = t / per_group;
-    const int first_m = g * p.group_m;
-    const int gsz = min(p.m_blocks - first_m, p.group_m);
-    const int mb = first_m + (t - g * per_group) % gsz;
+    const SplitTile tile = split_tile(p.raster, t);
+    const int mb = tile.m_block;
     const int m0 = mb * BM;
-    const int n0 = (t - g * per_group) / gsz * p.n_tile_stride;
+    const int n0 = tile.n_block * p.raster.n_tile_stride;
     long drow0 = m0;
     int b_row = 0, k_first = 0, k_blocks = (p.K + BK - 1) / BK;
     bool skip = false;
@@ -536,10 +531,7 @@ cudaError_t launch_gemm_split(const GemmArgs& a, const SplitPlan& plan, int sms,
     sp.M = a.M;
     sp.N = a.N;
     sp.K = a.K;
-    sp.n_tile_stride = swiglu ? plan.bn / 2 : plan.bn;
-    sp.m_blocks = (a.M + BM - 1) / BM;
-    sp.n_blocks = (a.N + sp.n_tile_stride - 1) / sp.n_tile_stride;
-    sp.group_m = 16;
+    sp.raster = split_raster(a, plan);
     sp.D = static_cast<const __nv_bfloat16*>(a.D);
     sp.ldd = a.ldd;
     sp.aux = static_cast<const __nv_bfloat16*>(a.aux);
@@ -551,7 +543,7 @@ cudaError_t launch_gemm_split(const GemmArgs& a, const SplitPlan& plan, int sms,
     sp.k_end = a.grouped.k_end;
     sp.error_flag = a.error_flag;
     sp.wait_limit_ns = a.wait_limit_ns ? a.wait_limit_ns : 4000000000ull;
-    const int tiles = sp.m_blocks * sp.n_blocks * (grouped_k ? static_cast<int>(groups) : 1);
+    const int tiles = sp.raster.m_blocks * sp.raster.n_blocks * (grouped_k ? static_cast<int>(groups) : 1);
     // Ring depth: all of shared memory when every CTA can have an SM of its own, half of it (two
     // CTAs per SM) otherwise; never more stages than the CTA has k-steps.
     const int kb = ((a.K + BK - 1) / BK + plan.splits - 1) / plan.splits;

@@ -1170,7 +1170,7 @@ int sm_count() {
 uint64_t gemm_launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 namespace {
-// Tile variant and raster of a problem: what launch_gemm_bf16 runs and tile_schedule reports.
+// Tile variant and raster of a problem that plan_split leaves to the persistent kernel.
 struct Plan {
     bool pair, wide;
     int tile_m;
@@ -1342,6 +1342,19 @@ SplitPlan plan_split(const GemmArgs& a, int sms) {
 int tile_schedule(const GemmArgs& a, int sms, int* tiles, int max_tiles) {
     if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.grouped.m_block_group != nullptr || a.grouped.k_begin != nullptr)
         return -1;
+    if (const SplitPlan sp = plan_split(a, sms); sp.bn != 0) {
+        if (!split_accepts(a, sp))
+            return -1;
+        const SplitRaster r = split_raster(a, sp);
+        for (int t = 0; t < r.m_blocks * r.n_blocks && t < max_tiles; ++t) {
+            const SplitTile tl = split_tile(r, t);
+            tiles[4 * t + 0] = tl.m_block * BM;
+            tiles[4 * t + 1] = tl.n_block * r.n_tile_stride;
+            tiles[4 * t + 2] = BM;
+            tiles[4 * t + 3] = r.n_tile_stride;
+        }
+        return r.m_blocks * r.n_blocks;
+    }
     KParams kp{};
     const Plan pl = plan_tiles(a, &kp, sms);
     for (int t = 0; t < kp.num_tiles && t < max_tiles; ++t) {

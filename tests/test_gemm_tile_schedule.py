@@ -51,9 +51,40 @@ def test_rotation_starts_with_the_asked_row_block_and_keeps_column_sweeps_togeth
 def test_automatic_variant_picks_the_wide_tile_only_for_large_dense_problems():
     assert schedule(32768, 8192, 8192)[0][2] == 512
     assert schedule(32768, 8192, 1024)[0][2] == 256     # short K loop: epilogue would show
-    assert schedule(512, 8192, 8192)[0][2] == 256       # M below 1024
-    assert schedule(2048, 1024, 8192)[0][2] == 256      # too few tiles for 74 CTA pairs
-    assert schedule(128, 1024, 8192)[0][2] == 128
+    assert schedule(512, 8192, 8192)[0][2] == 256       # 64 tiles for 74 CTA pairs, 32 of the wide ones
+    assert schedule(4096, 4096, 2048)[0][2] == 256      # half as many tiles fill the waves worse
+
+
+def test_problems_of_one_wave_go_to_the_small_tiles():
+    assert schedule(2048, 1024, 8192)[0][2:] == (128, 256)
+    assert schedule(128, 1024, 8192)[0][2:] == (128, 128)
+    # one row of tiles, however many
+    assert schedule(128, 65536, 512)[0][2] == 128
+    # asked for by name
+    assert schedule(300, 264, 200, variant=64 + 2)[0][2:] == (128, 64)
+    assert schedule(300, 264, 200, variant=256 + 4, epilogue=EPI_SWIGLU)[0][2:] == (128, 128)
+
+
+def test_a_small_tile_that_the_kernel_does_not_have_has_no_schedule():
+    lib = _lib.load()
+    a = GemmArgs()
+    a.M, a.N, a.K, a.variant = 1024, 1024, 1024, 64 + 3
+    buf = (C.c_int * 16)()
+    assert lib.megray_gemm_tile_schedule(C.byref(a), 148, buf, 4) == -1
+
+
+@pytest.mark.parametrize("variant", [64 + 1, 64 + 4, 128 + 8, 256 + 1])
+@pytest.mark.parametrize("M,N", [(1, 8), (129, 72), (4096, 264), (2048 + 128, 1000), (16 * 128 + 1, 65)])
+@pytest.mark.parametrize("epilogue", [EPI_STORE, EPI_SWIGLU])
+def test_small_tiles_cover_the_output_exactly_once(variant, M, N, epilogue):
+    tile_n = (variant & ~63) // (2 if epilogue == EPI_SWIGLU else 1)
+    tiles = schedule(M, N, 4096, variant, epilogue)
+    assert all(t[2] == 128 and t[3] == tile_n for t in tiles)
+    want = {(128 * i, tile_n * j) for i in range(-(-M // 128)) for j in range(-(-N // tile_n))}
+    assert len(tiles) == len(want) and {t[:2] for t in tiles} == want
+    # 16 row blocks are swept over all columns before the next ones
+    first = tiles[: min(16, -(-M // 128)) * -(-N // tile_n)]
+    assert max(t[0] for t in first) < 16 * 128
 
 
 def test_grouped_problems_have_no_host_schedule():
