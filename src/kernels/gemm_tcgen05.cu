@@ -1411,6 +1411,16 @@ cudaError_t launch_gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
         return cudaErrorInvalidValue;
     if (a.a_ready != nullptr && (kp.rows_per_flag % BM))
         return cudaErrorInvalidValue;
+    // A grouped-K problem stacks one [M, N] result per group; rows that a tile has past M would land in
+    // the next group's result, so such shapes (M not a multiple of the tile) leave through the guarded
+    // row-segment stores.  What those cannot do is refused here, before the small tiles, which could do
+    // more of it, are considered: whether a call is accepted does not depend on its size.
+    int epi = a.epilogue;
+    if (grouped_k && (a.M % tile_m) && epi != EPI_PUSH && epi != EPI_STORE_ROWS) {
+        if (epi != EPI_STORE || (a.N % 8))
+            return cudaErrorInvalidValue;
+        epi = EPI_STORE_ROWS;
+    }
 
     if (const SplitPlan sp = plan_split(a, sms); sp.bn != 0)
         return launch_gemm_split(a, sp, sms, stream);
@@ -1452,21 +1462,11 @@ cudaError_t launch_gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
         if (lim < workers)
             workers = lim > 0 ? lim : 1;
     }
-    // Output maps of the TMA-store epilogues.  A grouped-K problem stacks one [M, N] result per
-    // group; rows that a tile has past M would land in the next group's result, so such shapes
-    // (M not a multiple of the tile) leave through the guarded row-segment stores instead.
-    int epi = a.epilogue;
+    // Output maps of the TMA-store epilogues.
     const uint64_t out_rows = static_cast<uint64_t>(a.M) * (grouped_k ? groups : 1);
-    if (epi == EPI_STORE && grouped_k && (a.M % tile_m)) {
-        if (a.N % 8)
-            return cudaErrorInvalidValue;
-        epi = EPI_STORE_ROWS;
-    }
     if (epi == EPI_PUSH || epi == EPI_STORE_ROWS) {
         maps.d = maps.du = maps.d2 = maps.a;  // not used by these epilogues
     } else {
-        if (grouped_k && (a.M % tile_m))
-            return cudaErrorInvalidValue;
         ok = make_out_map(&maps.d, a.D, a.N, out_rows, a.ldd, epi == EPI_STORE_F32);
         maps.du = maps.d2 = maps.d;
         if (ok && (epi == EPI_SWIGLU || epi == EPI_DSWIGLU)) {

@@ -71,13 +71,15 @@ def test_row_segment_store_epilogue(M, N, K, variant):
     close(out, a.float() @ b.float().t())
 
 
-def test_accumulate():
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("M,N,K", [(256, 512, 128), (300, 264, 200), (520, 1000, 72)])
+def test_accumulate(M, N, K, variant):
     from megray_b200.ops import EPI_ACCUM, gemm
 
     torch.manual_seed(2)
-    a, b, d = mk(256, 128), mk(512, 128), mk(256, 512)
+    a, b, d = mk(M, K), mk(N, K), mk(M, N)
     d0 = d.clone()
-    gemm(a, b, d, epilogue=EPI_ACCUM)
+    gemm(a, b, d, epilogue=EPI_ACCUM, variant=variant)
     close(d, a.float() @ b.float().t() + d0.float())
 
 
@@ -101,7 +103,8 @@ def test_swiglu_and_its_derivative(variant):
     close(dgu, torch.cat([g.grad, u.grad], 1))
 
 
-def test_grouped_rows_pick_their_expert_weights():
+@pytest.mark.parametrize("variant", [0, 1])
+def test_grouped_rows_pick_their_expert_weights(variant):
     from megray_b200.ops import gemm
 
     torch.manual_seed(4)
@@ -111,7 +114,7 @@ def test_grouped_rows_pick_their_expert_weights():
     x, w = mk(M, K), mk(E * N, K)
     out = torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16)
     gemm(x, w, out, n=N, m_block_group=torch.tensor(blocks, device="cuda", dtype=torch.int32),
-         group_rows_b=N, groups=E)
+         group_rows_b=N, groups=E, variant=variant)
     torch.cuda.synchronize()
     for i, e in enumerate(blocks):
         rows = slice(128 * i, 128 * (i + 1))
@@ -164,3 +167,21 @@ def test_split_k_matches_the_plain_product(M, N, K, splits, a_mn, b_mn):
     gemm_split_k(a, b, out, splits, a_mn=a_mn, b_mn=b_mn)
     want = (a.float().t() if a_mn else a.float()) @ (b.float() if b_mn else b.float().t())
     close(out, want, tol=1e-2)
+
+
+@pytest.mark.parametrize("T", [256, 8192])
+def test_grouped_k_shapes_are_refused_at_every_size(T):
+    """One result per group is stacked on the next: rows past M of a float32 or unaligned result would have
+    nowhere to go on the 256-row tile."""
+    from megray_b200.ops import EPI_STORE_F32, gemm
+
+    kb = torch.tensor([0, T // 2], device="cuda", dtype=torch.int32)
+    ke = torch.tensor([T // 2, T], device="cuda", dtype=torch.int32)
+    for M in (384, 384 + 256 * 40):
+        dy, x = mk(T, M), mk(T, 256)
+        kw = dict(a_mn=True, b_mn=True, k_begin=kb, k_end=ke, groups=2)
+        with pytest.raises(RuntimeError):
+            gemm(dy, x, epilogue=EPI_STORE_F32, **kw)
+        with pytest.raises(RuntimeError):
+            gemm(dy, x, torch.empty(2 * M, 16, device="cuda", dtype=torch.bfloat16), n=12, **kw)
+        close(gemm(dy, x, **kw)[M:], dy[T // 2:].float().t() @ x[T // 2:].float())
