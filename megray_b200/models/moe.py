@@ -80,37 +80,40 @@ class MoELayer:
 
     def _native_args(self):
         """Argument block of the native passes for this call with what both of them use; None with a
-        communicator, or when a weight is not the contiguous matrix they take."""
+        communicator, or when a tensor is not the contiguous matrix they take."""
         ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
         if self.comm is not None:
             return None
-        a = _lib.MoEArgs(ep.T, ep.E, H, F, ep.capacity)
+        a, rows = _lib.MoEArgs(ep.T, ep.E, H, F, ep.capacity), ep.capacity
         a.w_gu, a.w_down = p = plain(self.w_gu, (ep.El * 2 * F, H)), plain(self.w_down, (ep.El * H, F))
-        if 0 in p:
+        a.x_perm, a.y_perm, a.gu, a.h = q = (plain(self.x_perm, (rows, H)), plain(self.y_perm, (rows, H)),
+                                             plain(self.gu, (rows, 2 * F)), plain(self.h, (rows, F)))
+        if 0 in p or 0 in q:
             return None
-        for name in ("x_perm", "y_perm", "gu", "h"):
-            setattr(a, name, getattr(self, name).data_ptr())
         for name in ("idx", "pos", "cursor", "send_base", "seg_begin", "seg_end", "seg_rows", "block_group", "w"):
             setattr(a, name, getattr(ep, name).data_ptr())
         a.error_flag = gemm_error_flag(self.h.device).data_ptr()
         return a
 
     def _native_forward_args(self):
-        a = self._native_args()
-        if a is not None:
-            a.out, a.counts, a.total = self.out.data_ptr(), self.ep.counts.data_ptr(), self.ep.total.data_ptr()
-        return a
+        a, ep = self._native_args(), self.ep
+        if a is None:
+            return None
+        a.out = p = plain(self.out, (ep.T, self.cfg.hidden))
+        a.counts, a.total = ep.counts.data_ptr(), ep.total.data_ptr()
+        return a if p else None
 
     def _native_backward_args(self):
         a, ep, F, H = self._native_args(), self.ep, self.cfg.ffn, self.cfg.hidden
         if a is None:
             return None
+        rows, f32 = ep.capacity, torch.float32
         a.g_gu, a.g_down = p = plain(self.g_gu, (ep.El * 2 * F, H)), plain(self.g_down, (ep.El * H, F))
-        if 0 in p:
-            return None
-        for name in ("dy_perm", "dx_perm", "dgu", "dx", "dw", "dlogits"):
-            setattr(a, name, getattr(self, name).data_ptr())
-        return a
+        a.dy_perm, a.dx_perm, a.dgu = q = (plain(self.dy_perm, (rows, H)), plain(self.dx_perm, (rows, H)),
+                                           plain(self.dgu, (rows, 2 * F)))
+        a.dx, a.dw, a.dlogits = r = (plain(self.dx, (ep.T, H)), plain(self.dw, (ep.T, 2), f32),
+                                     plain(self.dlogits, (ep.T, ep.E), f32))
+        return None if 0 in p or 0 in q or 0 in r else a
 
     # ------------------------------------------------------------------ forward / backward
     def forward(self, x: torch.Tensor, logits: torch.Tensor) -> torch.Tensor:

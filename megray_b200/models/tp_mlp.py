@@ -119,27 +119,27 @@ class TPMLPStack:
 
     def _native_args(self):
         """Argument block of the native passes for this call with what both of them use; None on several
-        ranks, or when a weight is not the contiguous matrix they take."""
+        ranks, or when a tensor is not the contiguous matrix they take."""
         if self.tp is not None or self.n != 1:
             return None
         T, d, f, L = self.Ts, self.cfg.d_model, self.cfg.ffn, len(self.layers)
         layers = (_lib.MLPLayer * L)()
         for l, w in enumerate(self.layers):
-            p = (plain(w.w_gu, (2 * f, d)), plain(w.w_down, (d, f)))
+            p = (plain(w.w_gu, (2 * f, d)), plain(w.w_down, (d, f)), plain(self.xg[l], (T, d)),
+                 plain(self.gu[l], (T, 2 * f)), plain(self.h[l], (T, f)), plain(self.inv_rms[l], (T,), torch.float32))
             if 0 in p:
                 return None
-            layers[l] = _lib.MLPLayer(*p, None, None, self.xg[l].data_ptr(), self.gu[l].data_ptr(),
-                                      self.h[l].data_ptr(), self.inv_rms[l].data_ptr())
+            layers[l] = _lib.MLPLayer(*p[:2], None, None, *p[2:])
         a = _lib.MLPArgs(L, T, d, f, layers)
         a.error_flag = gemm_error_flag(self.h[0].device).data_ptr()
         return a
 
     def _native_forward_args(self):
-        a = self._native_args()
-        if a is not None:
-            a.y = self.y.data_ptr()
-            a.xs[0], a.xs[1] = self.xs[0].data_ptr(), self.xs[1].data_ptr()
-        return a
+        a, row = self._native_args(), (self.Ts, self.cfg.d_model)
+        if a is None:
+            return None
+        a.y, a.xs[0], a.xs[1] = p = plain(self.y, row), plain(self.xs[0], row), plain(self.xs[1], row)
+        return None if 0 in p else a
 
     def _native_backward_args(self):
         a = self._native_args()
@@ -147,12 +147,15 @@ class TPMLPStack:
             return None
         T, d, f = self.Ts, self.cfg.d_model, self.cfg.ffn
         for l, w in enumerate(self.layers):
-            p = (plain(w.g_gu, (2 * f, d)), plain(w.g_down, (d, f)))
+            p = plain(w.g_gu, (2 * f, d)), plain(w.g_down, (d, f))
             if 0 in p:
                 return None
             a.layer[l].g_gu, a.layer[l].g_down = p
-        a.dgu, a.dn = self.dgu.data_ptr(), self.dn.data_ptr()
-        a.dres[0], a.dres[1] = self.dres[0].data_ptr(), self.dres[1].data_ptr()
+        row = (T, d)
+        a.dn, a.dres[0], a.dres[1] = p = plain(self.dn, row), plain(self.dres[0], row), plain(self.dres[1], row)
+        a.dgu = q = plain(self.dgu, (T, 2 * f))
+        if 0 in p or q == 0:
+            return None
         need = 0
         for split, M, N in ((a.split_down, d, f), (a.split_gu, 2 * f, d)):
             split.splits = s = pick_split_k(M, N, T)

@@ -78,3 +78,32 @@ def test_backward_into_gradients_that_are_no_plain_matrices():
         assert torch.equal(first(model.backward(dy)), dx)
         for got, g, t in zip((holder.g_gu, holder.g_down), want, wide):
             assert torch.equal(got, g) and bool((t[:, g.shape[1]:] == 7.0).all())
+
+
+def test_saved_activations_that_are_no_plain_matrices():
+    """Strided buffers in a model: op by op, the same result, and nothing beside them is written."""
+    for model, inputs, dy, holder in models():
+        want = model.forward(*inputs).clone()
+        model.backward(dy)
+        grad = holder.g_down.clone()
+        saved = {"h": model.h[0] if isinstance(model.h, list) else model.h, "dgu": model.dgu}
+        wide = {}
+        for name, t in saved.items():
+            wide[name] = torch.full((t.shape[0], t.shape[1] + 64), 7.0, device="cuda", dtype=torch.bfloat16)
+            view = wide[name][:, :t.shape[1]]
+            setattr(model, name, [view] if name == "h" and isinstance(model.h, list) else view)
+        assert model._native_forward_args() is None and model._native_backward_args() is None
+        assert torch.equal(model.forward(*inputs), want)
+        model.backward(dy)
+        assert float((holder.g_down.double() - grad.double()).norm()) <= 2.0 ** -8 * float(grad.double().norm())
+        for name, t in saved.items():
+            assert bool((wide[name][:, t.shape[1]:] == 7.0).all()) and not bool((wide[name][:, :t.shape[1]] == 7.0).all())
+
+
+def test_buffers_are_asked_for_their_size():
+    """A saved activation of another size is nothing the native passes write to."""
+    for model, inputs, _, _ in models():
+        h = model.h[0] if isinstance(model.h, list) else model.h
+        for other in (h[:-1], h[1:], h.float(), torch.cat([h, h])):
+            setattr(model, "h", [other] if isinstance(model.h, list) else other)
+            assert model._native_forward_args() is None
