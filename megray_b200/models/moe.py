@@ -26,6 +26,9 @@ from ..parallel.expert_parallel import ExpertParallelOps
 from ..ops._stream import raw_stream
 from ._native import plain
 
+# the steps of ExpertParallelOps that the native passes make themselves
+_EP_STEPS = frozenset(("route", "plan", "zero_pads", "dispatch", "barrier", "combine", "combine_dw", "route_bwd"))
+
 
 @dataclass
 class MoEConfig:
@@ -80,9 +83,10 @@ class MoELayer:
 
     def _native_args(self):
         """Argument block of the native passes for this call with what both of them use; None with a
-        communicator, or when a tensor is not the contiguous matrix they take."""
+        communicator or an ``ep`` that routes or exchanges in its own way, or when a tensor is not the
+        contiguous matrix they take."""
         ep, F, H = self.ep, self.cfg.ffn, self.cfg.hidden
-        if self.comm is not None:
+        if self.comm is not None or type(ep) is not ExpertParallelOps or not _EP_STEPS.isdisjoint(ep.__dict__):
             return None
         a, rows = _lib.MoEArgs(ep.T, ep.E, H, F, ep.capacity), ep.capacity
         a.w_gu, a.w_down = p = plain(self.w_gu, (ep.El * 2 * F, H)), plain(self.w_down, (ep.El * H, F))

@@ -142,7 +142,9 @@ class TPMLPStack:
         return None if 0 in p else a
 
     def _native_backward_args(self):
-        a = self._native_args()
+        # (a model with a weight-gradient product of its own runs it)
+        own = type(self)._wgrad is not TPMLPStack._wgrad or "_wgrad" in self.__dict__
+        a = None if own else self._native_args()
         if a is None:
             return None
         T, d, f = self.Ts, self.cfg.d_model, self.cfg.ffn

@@ -107,3 +107,37 @@ def test_buffers_are_asked_for_their_size():
         for other in (h[:-1], h[1:], h.float(), torch.cat([h, h])):
             setattr(model, "h", [other] if isinstance(model.h, list) else other)
             assert model._native_forward_args() is None
+
+
+def test_steps_of_its_own_are_run():
+    """A weight-gradient product, routing or exchange that a program puts in place of the library's."""
+    from megray_b200.models import TPMLPStack
+    from megray_b200.parallel.expert_parallel import ExpertParallelOps
+
+    seen = []
+
+    class OwnProduct(TPMLPStack):
+        def _wgrad(self, a_t, b_t, out):
+            seen.append("wgrad")
+            super()._wgrad(a_t, b_t, out)
+
+    class OwnRouting(ExpertParallelOps):
+        def route(self, logits):
+            seen.append("route")
+            super().route(-logits)
+
+    (mlp, inputs, dy, _), (moe, (x, logits), _, _) = models()
+    own = OwnProduct(mlp.cfg)
+    assert own._native_forward_args() is not None  # it has no weight gradient
+    own.forward(*inputs)
+    own.backward(dy)
+    assert seen == ["wgrad"] * 2
+    moe.ep = OwnRouting(None, moe.cfg.tokens, moe.cfg.hidden, moe.cfg.experts, moe.cfg.capacity_factor)
+    moe.forward(x, logits)
+    assert seen[2:] == ["route"] and torch.equal(moe.ep.idx.long(), (-logits).topk(2, dim=1).indices)
+    moe.ep = ExpertParallelOps(None, moe.cfg.tokens, moe.cfg.hidden, moe.cfg.experts, moe.cfg.capacity_factor)
+    assert moe._native_forward_args() is not None
+    combine = moe.ep.combine
+    moe.ep.combine = lambda *a, **kw: (seen.append("combine"), combine(*a, **kw))
+    moe.forward(x, logits)
+    assert seen[3:] == ["combine"]
