@@ -30,7 +30,6 @@
 // fused tensor-parallel and expert-parallel entry points.
 #include "gemm_device.cuh"
 
-#include <atomic>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -1043,8 +1042,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 
 // ------------------------------------------------------------------ host side
 
-std::atomic<uint64_t> g_launches{0};
-
 // Launches one instantiation.  `workers` = CTAs (single) or CTA pairs (pair) wanted at most;
 // the pair variant is additionally capped by what the device can co-schedule as 2-CTA clusters.
 template <int MODE, bool A_MN, bool B_MN, int EPI>
@@ -1109,7 +1106,6 @@ cudaError_t launch_t(const Maps& maps, const KParams& kp, int workers, cudaStrea
     cfg.attrs = attrs;
     cfg.numAttrs = 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, maps.a, maps.b, maps.d, maps.du, maps.d2, kp);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
     count_launch();
     return e;
 }
@@ -1165,11 +1161,6 @@ int sm_count() {
     return n;
 }
 
-}  // namespace
-
-uint64_t gemm_launch_count() { return g_launches.load(std::memory_order_relaxed); }
-
-namespace {
 // Tile variant and raster of a problem that plan_split leaves to the persistent kernel.
 struct Plan {
     bool pair, wide;

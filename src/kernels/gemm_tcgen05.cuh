@@ -110,8 +110,5 @@ cudaError_t launch_gemm_bf16(const GemmArgs& args, cudaStream_t stream);
 // worker t mod workers, on the small-tile kernel on cluster t.  Needs no GPU.
 int tile_schedule(const GemmArgs& args, int sms, int* tiles, int max_tiles);
 
-// Number of kernels this module has launched since load (for launch accounting).
-uint64_t gemm_launch_count();
-
 }  // namespace gemm
 }  // namespace mgk
