@@ -9,7 +9,9 @@
 //
 // Three variants of one kernel template:
 //   single : one CTA per tile, tile 128 x 256 x 64, tcgen05.mma.cta_group::1 (M = 128),
-//            4-stage ring of 48 KB.  Used for grouped (per-expert) row blocks.
+//            4-stage ring of 48 KB.  Used for rows grouped by expert while a group has few
+//            128-row blocks, and for at most 128 rows where the small tiles (gemm_split.cu)
+//            do not apply (fused calls, a limit on the SMs).
 //   pair   : a cluster of two CTAs per 256 x 256 tile, tcgen05.mma.cta_group::2 (M = 256)
 //            issued by the leader CTA; each CTA stages its own 128 rows of A and its own
 //            128 rows of B (so B is read from shared memory once per pair), 6-stage ring
@@ -132,8 +134,8 @@ struct Tile {
     bool skip;     // nothing to do (padding block of a grouped problem)
 };
 
-// Row blocks of a grouped problem on a tile of more than 128 rows: consecutive 128-row blocks of
-// one group are put together, up to a full tile; padding blocks are left out.  One entry per tile
+// Row blocks of a grouped problem on the 256-row tile: consecutive 128-row blocks of one group are
+// put together, up to a full tile; padding blocks are left out.  One entry per tile
 // row: first block | (blocks - 1) << 14.
 struct RowTiles {
     const uint16_t* list;  // null = tile rows are TILE_M rows apart
@@ -552,9 +554,9 @@ __device__ __forceinline__ void all_gather_warps(const FuseArgs& f, uint64_t lim
     }
 }
 
-// Fills the row-tile list of a grouped problem (one warp; R blocks per tile at most).
-template <int R>
+// Fills the row-tile list of a grouped problem (one warp; two blocks per tile at most).
 __device__ __forceinline__ void build_row_tiles(const KParams& p, uint16_t* list, int* count, int lane) {
+    constexpr int R = 2;
     const int blocks = (p.M + BM - 1) / BM;
     int n = 0, prev = -2, prev_pos = 0;  // group of the block before this batch, its place in its run
     for (int b0 = 0; b0 < blocks; b0 += 32) {
@@ -620,13 +622,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     const uint32_t tfull0 = smem_u32(bars + 2 * STAGES);
     const uint32_t tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
-    constexpr bool ROW_TILES = C::TILE_M > BM && (EPI == EPI_STORE || EPI == EPI_SWIGLU || EPI == EPI_DSWIGLU);
+    constexpr bool ROW_TILES = MODE == MODE_PAIR && (EPI == EPI_STORE || EPI == EPI_SWIGLU || EPI == EPI_DSWIGLU);
     uint16_t* row_list = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + BAR_BYTES);
     int* row_count = reinterpret_cast<int*>(tmem_slot + 8);
     RowTiles rt{nullptr, 0};
     if (ROW_TILES && p.m_block_group != nullptr) {
         if (warp == 2)
-            build_row_tiles<C::TILE_M / BM>(p, row_list, row_count, lane);
+            build_row_tiles(p, row_list, row_count, lane);
         rt.list = row_list;
     }
 
@@ -1170,10 +1172,10 @@ Plan plan_tiles(const GemmArgs& a, KParams* kpp, int sms) {
     KParams& kp = *kpp;
     const bool grouped_m = a.grouped.m_block_group != nullptr;
     const bool grouped_k = a.grouped.k_begin != nullptr;
-    // A CTA pair per tile unless rows are grouped in 128-row blocks (per-expert
-    // forward/backward), which need the 128-row tile.  Large dense problems take the
-    // 512-row tile: less operand traffic per FLOP, at the price of an epilogue that is
-    // only half hidden, which a long K loop amortises.
+    // A CTA pair per tile, except for at most 128 rows and for rows grouped in 128-row blocks of
+    // which a group has few.  Dense problems take the 256- or the 512-row tile by estimated time:
+    // the larger one moves less operand traffic per FLOP, at the price of an epilogue that is only
+    // half hidden, which a long K loop amortises, and of fewer tiles to fill the waves with.
     // MEGRAY_GEMM_VARIANT stands in for variant 0 (a tuning and test aid)
     static const int env_variant = [] {
         const char* e = getenv("MEGRAY_GEMM_VARIANT");
@@ -1183,17 +1185,23 @@ Plan plan_tiles(const GemmArgs& a, KParams* kpp, int sms) {
     Plan pl;
     pl.pair = variant != 1 && a.M > 128;
     if (grouped_m) {
-        // Tiles of two 128-row blocks of one group (row-tile list) once a group has several blocks; the
-        // capacity M / groups is an upper bound of a group's rows.  8 experts of 4096 rows, 4096 ->
-        // 14336: SwiGLU product 6.64 ms on the 128-row tile, 5.59 on the 256-row tile; 16 experts of 250
-        // rows, down product: 0.66 and 0.48 ms; 16 of 31 rows: 0.31 and 0.37 ms.  The 512-row tile is
-        // no better than the 256-row one and loses up to a quarter on short groups.
+        // Tiles of two 128-row blocks of one group (row-tile list) once a group has several blocks.  How many
+        // it has is known on the device only; the capacity M / groups stands in for it, which is the mean
+        // with its padding: one group may hold far more and the others far fewer.  The groups with many
+        // blocks are then the work, so the line holds for skewed routing as well.  The four grouped products
+        // of a layer together, 128-row / 256-row tiles, in microseconds: 8 experts, 4096 -> 14336, capacity
+        // 448: 2050 / 1797 with even routing, 2087 / 1836 with 6, 4, 3, 2, 1, 1, 1, 1 blocks, 2209 / 1755
+        // with 8 and seven times 2; capacity 5248: 21458 / 17853 even, 21307 / 17849 with two experts of
+        // 128 blocks and six of one.  16 experts, 1024 -> 2048, capacity 768: 298 / 277 even, 310 / 292
+        // skewed; capacity 288: 248 / 265 even, 175 / 221 skewed.  64 experts, 2048 -> 3584, capacity 448:
+        // 1993 / 1926 even, 2264 / 2200 skewed, although the dSwiGLU product alone loses there (463 / 524).
+        // The 512-row tile is no better than the 256-row one and loses up to a quarter on short groups.
         const bool can = (a.epilogue == EPI_STORE || a.epilogue == EPI_SWIGLU || a.epilogue == EPI_DSWIGLU) &&
                          (a.M + BM - 1) / BM <= MAX_ROW_TILES && a.m_rot == 0;
         const long rows = a.M / (a.grouped.groups > 0 ? a.grouped.groups : 1);
         pl.pair = pl.pair && can && (variant != 0 || rows >= 384);
     }
-    pl.wide = pl.pair && variant == 3;
+    pl.wide = pl.pair && variant == 3 && !grouped_m;
     if (pl.pair && variant == 0 && !grouped_m && a.epilogue != EPI_DSWIGLU) {
         // (the dSwiGLU epilogue reads and writes four values per accumulator element; it needs
         // the next tile's main loop to hide behind: 12.9-13.2 ms on the pair tile against
@@ -1264,13 +1272,14 @@ Plan plan_tiles(const GemmArgs& a, KParams* kpp, int sms) {
 
 // Whether a problem goes to the small-tile / cluster split-K kernel, and with which tile.
 //
-// Only problems whose 128 x 256 tiles fit the chip in one wave are considered: there the persistent
-// kernel leaves SMs idle or, with few k-steps, is all prologue and epilogue (296 x 328 x 456: 9.6 ->
-// 6.1 us; 128 x 8192 x 28672: 176 -> 83 us; 1024 x 1024 x 4096: 24.6 -> 13.3 us); with more tiles the
-// CTA-pair kernel moves less data per FLOP and wins.  Within them a plan is chosen by an estimate
-// whose constants (microseconds) were fitted to 90 shapes from 128 x 256 x 256 to 4096 x 1024 x 16384:
-// launch 1.2 and 3.0 for each wave of CTAs; a k-step by tile width with up to half of the SMs in use, with all of them, and with
-// two CTAs on each; the epilogue and the exchange of the partials by tile width.
+// Considered are problems of at most 128 rows, and those whose 128 x 256 tiles fit the chip in one
+// wave or overfill it by a twelfth: there the persistent kernel leaves SMs idle or, with few k-steps,
+// is all prologue and epilogue (296 x 328 x 456: 9.6 -> 6.1 us; 128 x 8192 x 28672: 176 -> 83 us;
+// 1024 x 1024 x 4096: 24.6 -> 13.3 us); with more tiles the CTA-pair kernel moves less data per FLOP
+// and wins.  Within them a plan is chosen by an estimate whose constants (microseconds) were fitted to
+// 90 shapes from 128 x 256 x 256 to 4096 x 1024 x 16384: launch 1.2 and 3.0 for each wave of CTAs; a
+// k-step by tile width with up to half of the SMs in use, with all of them, and with two CTAs on each;
+// the epilogue and the exchange of the partials by tile width.
 SplitPlan plan_split(const GemmArgs& a, int sms) {
     const bool swiglu = a.epilogue == EPI_SWIGLU;
     const bool grouped_m = a.grouped.m_block_group != nullptr, grouped_k = a.grouped.k_begin != nullptr;
