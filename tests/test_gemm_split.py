@@ -1,32 +1,10 @@
-"""The small-tile / cluster split-K kernel against float64 at
-the sizes where they can go wrong: edges of tiles, remainders of K, more CTAs than k-steps, every
-operand layout and epilogue."""
+"""The small-tile / cluster split-K kernel against float64 at the sizes where it can go wrong: edges of
+tiles, remainders of K, more CTAs than k-steps, every operand layout and epilogue."""
 import pytest
 import torch
+from gemm_check import BLOCKS, check, check_dswiglu, mk, product
 
 pytestmark = pytest.mark.gpu
-
-
-def mk(r, c, scale=0.5):
-    return (torch.randn(r, c, device="cuda") * scale).to(torch.bfloat16)
-
-
-def product(a, b, a_mn, b_mn):
-    """(A B^T, |A| |B|^T) in float64."""
-    a, b = a.double(), b.double()
-    a, b = (a.t() if a_mn else a), (b if b_mn else b.t())
-    return a @ b, a.abs() @ b.abs()
-
-
-def check(got, want, mass, k, rounded=True):
-    """float32 sums of k products in any order are within k * 2^-24 of the sum of their magnitudes
-    (twice that here); a bf16 result is rounded once more, by at most 2^-8 of its value."""
-    from megray_b200.ops import gemm_error_flag
-
-    torch.cuda.synchronize()
-    assert int(gemm_error_flag().item()) == 0
-    bound = mass * (k * 2.0 ** -23) + (want.abs() * 2.0 ** -8 if rounded else 0) + 1e-30
-    assert bool(((got.double() - want).abs() <= bound).all())
 
 
 PLANS = [64 + 1, 64 + 2, 64 + 8, 128 + 1, 128 + 4, 128 + 8, 256 + 1, 256 + 2, 256 + 8]
@@ -68,12 +46,7 @@ def test_swiglu_and_its_derivative(variant, M, F, K):
     dy, wd = mk(M, K), mk(K, F, 0.1)
     dgu = gemm(dy, wd, b_mn=True, epilogue=EPI_DSWIGLU, aux=gu, n=F, variant=variant)
     dh, mass = product(dy, wd, False, True)
-    g, u = gu[:, :F].double(), gu[:, F:].double()
-    s = torch.sigmoid(g)
-    want = torch.cat([dh * u * (s + g * s * (1 - s)), dh * g * s], 1)
-    # the factors come from rounded values that both sides read; they are formed in float32 (16 * 2^-23)
-    scale = torch.cat([u.abs() * (s + g.abs() * s * (1 - s)), (g * s).abs()], 1)
-    check(dgu, want, scale * torch.cat([mass, mass], 1), K + 16)
+    check_dswiglu(dgu, gu, dh, mass, K)
 
 
 def test_a_shape_the_kernel_does_not_take_is_refused():
@@ -83,14 +56,6 @@ def test_a_shape_the_kernel_does_not_take_is_refused():
     for variant in (64 + 3, 64 + 16, 192 + 1):
         with pytest.raises(RuntimeError):
             gemm(a, b, variant=variant)
-
-
-BLOCKS = [
-    [0, 0, 0, 1, -1, 2, 2, 2, 2, 2, -1, -1],
-    [1] * 31 + [0] * 3 + [2] * 34 + [-1] * 3,  # runs across the 32-block batches of the list's builder
-    [-1, -1, 2],
-    [-1, -1],
-]
 
 
 @pytest.mark.parametrize("variant", [64 + 2, 256 + 1])
@@ -114,6 +79,30 @@ def test_grouped_rows(variant, blocks):
         else:
             check(out[r], *product(x[r], w[e * N:(e + 1) * N], False, False), K)
             check(gu[r], *product(x[r], wgu[e * 2 * N:(e + 1) * 2 * N], False, False), K)
+
+
+@pytest.mark.parametrize("variant", [64 + 4, 128 + 1, 256 + 2])
+@pytest.mark.parametrize("blocks", BLOCKS)
+def test_grouped_rows_against_transposed_weights(variant, blocks):
+    from megray_b200.ops import EPI_DSWIGLU, gemm
+
+    torch.manual_seed(6)
+    E, N, K, M = 3, 264, 192, 128 * len(blocks)
+    groups = dict(m_block_group=torch.tensor(blocks, device="cuda", dtype=torch.int32), groups=E, variant=variant,
+                  group_rows_b=K)
+    dy, w, gu = mk(M, K), mk(E * K, N, 0.1), mk(M, 2 * N)
+    out = torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm(dy, w, out, b_mn=True, n=N, **groups)
+    dgu = torch.full((M, 2 * N), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm(dy, w, dgu, b_mn=True, epilogue=EPI_DSWIGLU, aux=gu, n=N, **groups)
+    for i, e in enumerate(blocks):
+        r = slice(128 * i, 128 * (i + 1))
+        if e < 0:
+            assert all(bool((t[r] == 7.0).all()) for t in (out, dgu))
+        else:
+            dh, mass = product(dy[r], w[e * K:(e + 1) * K], False, True)
+            check(out[r], dh, mass, K)
+            check_dswiglu(dgu[r], gu[r], dh, mass, K)
 
 
 @pytest.mark.parametrize("variant", [64 + 4, 128 + 2])
