@@ -77,7 +77,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--no-cublas", action="store_true")
     ap.add_argument("--epilogue", type=int, default=0, help="0 = per-lane stores, 5 = row segments through smem")
-    ap.add_argument("--variant", type=int, default=0, help="0 = automatic, 1 = single-CTA 128x256 tile, 2 = CTA-pair 256x256 tile, 3 = CTA-pair 512x256 tile")
+    ap.add_argument("--variant", type=int, default=0, help="0 = automatic, 1 = single-CTA 128x256 tile, 2 = CTA-pair 256x256 tile, 3 = CTA-pair 512x256 tile, columns + splits (64, 128 or 256, plus 1, 2, 4 or 8) = 128-row tile, K loop shared by a cluster")
     ap.add_argument("--split-k", default="", help="comma-separated K-range counts to time as extra candidates "
                                                     "(plain layouts; 1 = no split)")
     ap.add_argument("--sustain", type=float, default=0.0,

@@ -1225,8 +1225,14 @@ Plan plan_tiles(const GemmArgs& a, KParams* kpp, int sms) {
             const double waves_pair = static_cast<double>((tiles_pair + workers - 1) / workers);
             const double step = swiglu ? 0.385 : 0.345, tail = swiglu ? 6.0 : 1.2;
             const double tile_pair = step * kb > 2.9 ? step * kb : 2.9, tile_wide = 0.67 * kb + tail > 4.5 ? 0.67 * kb + tail : 4.5;
-            // Products of many waves run at the power limit, where what the tile does not read counts too:
-            // with the pair tile for K = 3584 the step of 8192/3584 on 32768 tokens was 2 % slower.
+            // Products of many waves run at the power limit, where what the tile does not read counts too.
+            // 32768 x 8192 alone for 3 s at that limit, pair / wide tile in milliseconds: K = 3072 1.241 /
+            // 1.260, 3584 1.441 / 1.460, 4096 1.650 / 1.668, 8192 3.398 / 3.268; SwiGLU 32768 x 3584 x 8192
+            // 3.010 / 2.958.  Alone the wide tile gains from K = 8192 on; the line lies lower because with
+            // the pair tile for K = 3584 the whole step of 8192/3584 on 32768 tokens was 2 % slower.  What
+            // that costs: SwiGLU 4096 x 7168 x 4096 takes 0.406 ms, 0.375 on the pair tile.  With fewer
+            // waves the factor is for ragged K: 1544 x 3080 x 5000 takes 56 us on the wide tile, 71 on the
+            // pair tile; where K is a multiple of 64 the two are within 3 % (4096 x 4096 x 4096 111 / 114).
             const double power = kb >= 48 && waves_pair > 8 ? 0.9 : kb >= 64 ? 0.97 : 1.0;
             pl.wide = (8.0 + waves_wide * tile_wide) * power < 6.6 + waves_pair * tile_pair;
         }
